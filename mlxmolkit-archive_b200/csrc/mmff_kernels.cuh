@@ -37,6 +37,7 @@
 #include <string>
 
 #include "mmff_terms.cuh"
+#include "mmff_terms32.cuh"
 #include "mmffb200.h"
 
 namespace mmffb {
@@ -139,7 +140,7 @@ __host__ __device__ __forceinline__ size_t al16(size_t x) { return (x + 15) & ~(
 constexpr int kStages = 4;         // rows of H in flight per warp (TMA ring)
 
 struct Layout {
-    size_t pos4, pos4d, x, g, dir, xo, dg, hp, hq, pxi, pc, pr, gbuf, cls, q, qf, mask, tab, red, rho, alpha,
+    size_t pos4, pos4d, x, g, dir, xo, dg, hp, hq, pxi, pc, pr, gbuf, cls, q, mask, tab, red, rho, alpha,
         ring, mbar, mat, total;
 };
 
@@ -166,7 +167,6 @@ __host__ __device__ inline Layout make_layout(int nmax, int nwarps, int hist_m, 
     L.gbuf = o; o = al16(o + (size_t)nwarps * nv * rs);
     L.cls = o; o = al16(o + (size_t)nmax * 4);
     L.q = o; o = al16(o + (size_t)nmax * 8);
-    L.qf = o; o = al16(o + (size_t)nmax * 4);
     L.mask = o; o = al16(o + 2 * (size_t)nmax * ((nmax + 31) / 32) * 4);
     L.tab = o; o = al16(o + (size_t)max_classes * max_classes * 8);
     L.red = o; o = al16(o + 2 * (size_t)nwarps * 8 * as);
@@ -200,7 +200,6 @@ __host__ __device__ inline Layout make_eval_layout(int nmax, int nwarps, size_t 
     L.gbuf = o; o = al16(o + (size_t)nwarps * nv * rs);
     L.cls = o; o = al16(o + (size_t)nmax * 4);
     L.q = o; o = al16(o + (size_t)nmax * 8);
-    L.qf = o; o = al16(o + (size_t)nmax * 4);
     L.mask = o; o = al16(o + 2 * (size_t)nmax * ((nmax + 31) / 32) * 4);
     L.tab = o; o = al16(o + (size_t)max_classes * max_classes * 8);
     L.red = o; o = al16(o + 2 * (size_t)nwarps * 8 * as);
@@ -319,8 +318,7 @@ __device__ __forceinline__ float u2f(uint32_t u) { return __uint_as_float(u); }
 // Per-conformer molecule data staged in shared memory.
 struct MolSmem {
     const int *cls;        // non-bonded class per atom
-    const double *qa;      // partial charge per atom (FP64)
-    const float *qf;       // the same, float (FP32 pair math)
+    const double *qa;      // partial charge per atom (FP64; FP32 evaluations take it from pos4)
     const uint32_t *mask;  // N x W non-bonded-pair bit rows, then N x W 1-4 bit rows
     const float2 *tab;     // ncls x ncls (R*, eps)
 };
@@ -333,25 +331,18 @@ template <> __device__ __forceinline__ void ld3<float>(const float *p4, int a, f
     x = v.x; y = v.y; z = v.z;
 }
 
-template <class R> __device__ __forceinline__ R pair_charge(const MolSmem &ms, int i, int j);
-template <> __device__ __forceinline__ float pair_charge<float>(const MolSmem &ms, int i, int j) {
-    return ms.qf[i] * ms.qf[j];
-}
-template <> __device__ __forceinline__ double pair_charge<double>(const MolSmem &ms, int i, int j) {
-    return qprod<double>(ms.qa[i], ms.qa[j]);
-}
-
 // Copy a molecule's bit rows, class table, classes and charges into shared memory.
 // IR (the FP32 instances): stage 1/R* in place of R*, the pair term's only use of R*.
+// pos4 (FP32 instances): its fourth component takes the atom's charge, read with the position.
 template <int NT, bool IR = false>
-__device__ __forceinline__ void stage_molecule(const Params &P, const MolV &m, int *cls, double *qa, float *qf,
+__device__ __forceinline__ void stage_molecule(const Params &P, const MolV &m, int *cls, double *qa, float *pos4,
                                                uint32_t *mask, float2 *tab) {
     const int N = m.n, W = (N + 31) >> 5;
     for (int a = threadIdx.x; a < N; a += NT) {
         cls[a] = __ldcg(P.b.atom_cls + m.atom_off + a);
         const double q = __ldcg(P.b.atom_q + m.atom_off + a);
         qa[a] = q;
-        qf[a] = (float)q;
+        if (IR) pos4[4 * a + 3] = (float)q;
     }
     const uint32_t *gm = P.b.pair_mask + m.mask_off;
     for (int k = threadIdx.x; k < 2 * N * W; k += NT) mask[k] = __ldcg(gm + k);
@@ -363,12 +354,216 @@ __device__ __forceinline__ void stage_molecule(const Params &P, const MolV &m, i
     }
 }
 
+// Warp sums of the forces on two rows, each to the buffer entry it belongs to: a butterfly
+// that halves the values a lane carries at every level (8 shuffles for 6 sums; the sum of each
+// value has the tree of a full butterfly, so the same bits).  gi2 may be null.
+__device__ __forceinline__ void scatter_rows(const float (&f)[3], const float (&k)[3], float *gi, float *gi2) {
+    const int lane = threadIdx.x & 31;
+    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+    float w[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) w[c] = (b4 ? k[c] : f[c]) + __shfl_xor_sync(0xffffffffu, b4 ? f[c] : k[c], 16);
+    const float xz = (b3 ? w[2] : w[0]) + __shfl_xor_sync(0xffffffffu, b3 ? w[0] : w[2], 8);
+    const float yy = w[1] + __shfl_xor_sync(0xffffffffu, w[1], 8);
+    float z = (b2 ? yy : xz) + __shfl_xor_sync(0xffffffffu, b2 ? xz : yy, 4);
+    z += __shfl_xor_sync(0xffffffffu, z, 2);
+    z += __shfl_xor_sync(0xffffffffu, z, 1);
+    float *dst = b4 ? gi2 : gi;
+    if ((lane & 3) == 0 && !(b3 && b2) && dst) {
+        dst += b2 ? 1 : (b3 ? 2 : 0);
+        *dst += z;
+    }
+}
+
+// The FP32 evaluation: energy (thread partial, not reduced) and -- if G -- per-warp gradient
+// buffers.  pos4: x, y, z and the charge of each atom; the class table holds 1/R*.
+template <class A, int NW, bool G>
+__device__ __forceinline__ A eval_terms32(const Params &P, const MolV &m, const float *pos4, float *gbuf,
+                                          const MolSmem &ms, int nv, int forms) {
+    using t32::V3;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int N = m.n;
+    A acc = A(0);
+    float *gw = gbuf + (size_t)warp * nv;
+    if (G) {
+        for (int k = lane; k < 3 * N; k += 32) gw[k] = 0.0f;
+        __syncwarp();
+    }
+    const uint4 *BR = reinterpret_cast<const uint4 *>(P.b.bonded);
+    const t32::Mode md(P.md);
+
+    for (int c = warp; c < m.bnch; c += NW) {
+        const uint4 r = __ldg(BR + m.boff + (size_t)c * 32 + lane);
+        const bool v = r.x != 0xffffffffu;
+        const int i = r.x & 0xffff, j = r.x >> 16;
+        V3 f;
+        if (v) {
+            acc += (A)t32::bond<G>(t32::at(pos4, i), t32::at(pos4, j), u2f(r.y), u2f(r.z),
+                                     (forms & t32::kBondApart) != 0, f);
+            if (G) t32::acc(gw + 3 * i, f);
+        }
+        if (G) {
+            __syncwarp();
+            if (v) t32::dec(gw + 3 * j, f);
+            __syncwarp();
+        }
+    }
+    for (int c = warp; c < m.anch; c += NW) {
+        const uint4 r = __ldg(BR + m.aoff + (size_t)c * 32 + lane);
+        const bool v = r.x != 0xffffffffu;
+        const int i = r.x & 0xffff, j = r.x >> 16, k = r.y & 0xffff;
+        const bool lin = (r.y >> 16) != 0;
+        V3 f0, f1, f2;
+        if (v) {
+            float s0;
+            acc += (A)t32::angle<G>(t32::at(pos4, i), t32::at(pos4, j), t32::at(pos4, k), u2f(r.z), u2f(r.w), lin, md,
+                                    s0, f0, f1, f2);
+            if (G) t32::accm(gw + 3 * i, s0, f0);
+        }
+        if (G) {
+            __syncwarp();
+            if (v) t32::dec(gw + 3 * j, f1);
+            __syncwarp();
+            if (v) t32::acc(gw + 3 * k, f2);
+            __syncwarp();
+        }
+    }
+    for (int c = warp; c < m.snch; c += NW) {
+        const uint4 r0 = __ldg(BR + m.soff + (size_t)c * 64 + lane);
+        const uint4 r1 = __ldg(BR + m.soff + (size_t)c * 64 + 32 + lane);
+        const bool v = r0.x != 0xffffffffu;
+        const int i = r0.x & 0xffff, j = r0.x >> 16, k = (int)r0.y;
+        V3 f0, f1, f2;
+        if (v) {
+            acc += (A)t32::strbend<G>(t32::at(pos4, i), t32::at(pos4, j), t32::at(pos4, k), u2f(r0.z), u2f(r0.w),
+                                      u2f(r1.x), u2f(r1.y), u2f(r1.z), md, (forms & t32::kStrbendApart) != 0, f0, f1, f2);
+            if (G) t32::acc(gw + 3 * i, f0);
+        }
+        if (G) {
+            __syncwarp();
+            if (v) t32::acc(gw + 3 * j, f1);
+            __syncwarp();
+            if (v) t32::acc(gw + 3 * k, f2);
+            __syncwarp();
+        }
+    }
+    for (int c = warp; c < m.onch; c += NW) {
+        const uint4 r = __ldg(BR + m.ooff + (size_t)c * 32 + lane);
+        const bool v = r.x != 0xffffffffu;
+        const int i = r.x & 0xffff, j = r.x >> 16, k = r.y & 0xffff, l = r.y >> 16;
+        V3 f0, f1, f2, f3;
+        if (v) {
+            float s0;
+            acc += (A)t32::oop<G>(t32::at(pos4, i), t32::at(pos4, j), t32::at(pos4, k), t32::at(pos4, l), u2f(r.z), md,
+                                  s0, f0, f1, f2, f3);
+            if (G) t32::accm(gw + 3 * i, s0, f0);
+        }
+        if (G) {
+            __syncwarp();
+            if (v) t32::dec(gw + 3 * j, f1);
+            __syncwarp();
+            if (v) t32::acc(gw + 3 * k, f2);
+            __syncwarp();
+            if (v) t32::acc(gw + 3 * l, f3);
+            __syncwarp();
+        }
+    }
+    for (int c = warp; c < m.tnch; c += NW) {
+        const uint4 r0 = __ldg(BR + m.toff + (size_t)c * 64 + lane);
+        const uint4 r1 = __ldg(BR + m.toff + (size_t)c * 64 + 32 + lane);
+        const bool v = r0.x != 0xffffffffu;
+        const int i = r0.x & 0xffff, j = r0.x >> 16, k = r0.y & 0xffff, l = r0.y >> 16;
+        V3 f0, f1, f2, f3;
+        if (v) {
+            acc += (A)t32::torsion<G>(t32::at(pos4, i), t32::at(pos4, j), t32::at(pos4, k), t32::at(pos4, l),
+                                      u2f(r0.z), u2f(r0.w), u2f(r1.x), (forms & t32::kTorsionApart) != 0, f0, f1, f2, f3);
+            if (G) t32::acc(gw + 3 * i, f0);
+        }
+        if (G) {
+            __syncwarp();
+            if (v) t32::acc(gw + 3 * j, f1);
+            __syncwarp();
+            if (v) t32::acc(gw + 3 * k, f2);
+            __syncwarp();
+            if (v) t32::acc(gw + 3 * l, f3);
+            __syncwarp();
+        }
+    }
+
+    // Non-bonded pairs, implicit from the staged bit rows and class table: rows i and i + NW per
+    // step, lanes over the columns, so two independent pair chains per lane and one scatter per
+    // column (a pair absent from the bit rows contributes nothing).
+    const int W = (N + 31) >> 5;
+    const uint32_t *pm = ms.mask, *p14 = ms.mask + (size_t)N * W;
+    const float4 *X = reinterpret_cast<const float4 *>(pos4);
+    const bool dd = m.diel == 2;
+    for (int i = warp; i < N - 1; i += 2 * NW) {
+        const int i2 = i + NW;
+        const bool has2 = i2 < N - 1;
+        const int ik = has2 ? i2 : i;
+        const float4 a = X[i], b = X[ik];
+        const float2 *ti = ms.tab + ms.cls[i] * m.ncls, *tk = ms.tab + ms.cls[ik] * m.ncls;
+        const uint32_t *mi = pm + i * W, *mk = pm + ik * W, *ni = p14 + i * W, *nk = p14 + ik * W;
+        float f[3] = {0.0f, 0.0f, 0.0f}, k[3] = {0.0f, 0.0f, 0.0f};
+        const int w2 = has2 ? (i2 + 1) >> 5 : W;   // the second row's first word
+        for (int wb = (i + 1) >> 5; wb < W; ++wb) {
+            const uint32_t wd = mi[wb], wd2 = wb >= w2 ? mk[wb] : 0u;
+            const bool b1 = (wd >> lane) & 1u, b2 = (wd2 >> lane) & 1u;
+            if (b1 || b2) {
+                const int j = 32 * wb + lane, cj = ms.cls[j];
+                const float2 t1 = ti[cj], t2 = tk[cj];
+                const float4 x = X[j];
+                float q1 = __fmul_rn(a.w, x.w), q2 = __fmul_rn(b.w, x.w);
+                if ((ni[wb] >> lane) & 1u) q1 = __fmul_rn(q1, 0.75f);
+                if ((nk[wb] >> lane) & 1u) q2 = __fmul_rn(q2, 0.75f);
+                const float dx1 = a.x - x.x, dy1 = a.y - x.y, dz1 = a.z - x.z;
+                const float dx2 = b.x - x.x, dy2 = b.y - x.y, dz2 = b.z - x.z;
+                float ev1, ee1, s1, ev2, ee2, s2;
+                t32::pair<G>(dx1, dy1, dz1, t1.x, t1.y, q1, dd, ev1, ee1, s1);
+                t32::pair<G>(dx2, dy2, dz2, t2.x, t2.y, q2, dd, ev2, ee2, s2);
+                if (b1) {
+                    acc += (A)ev1;
+                    acc += (A)ee1;
+                }
+                if (b2) {
+                    acc += (A)ev2;
+                    acc += (A)ee2;
+                }
+                if (G) {
+                    const float m1 = b1 ? s1 : 0.0f, m2 = b2 ? s2 : 0.0f;
+                    const float g2x = __fmul_rn(m2, dx2), g2y = __fmul_rn(m2, dy2), g2z = __fmul_rn(m2, dz2);
+                    f[0] = __fmaf_rn(m1, dx1, f[0]);
+                    f[1] = __fmaf_rn(m1, dy1, f[1]);
+                    f[2] = __fmaf_rn(m1, dz1, f[2]);
+                    k[0] = __fadd_rn(k[0], g2x);
+                    k[1] = __fadd_rn(k[1], g2y);
+                    k[2] = __fadd_rn(k[2], g2z);
+                    float *gj = gw + 3 * j;
+                    gj[0] = __fadd_rn(gj[0], -__fmaf_rn(m1, dx1, g2x));
+                    gj[1] = __fadd_rn(gj[1], -__fmaf_rn(m1, dy1, g2y));
+                    gj[2] = __fadd_rn(gj[2], -__fmaf_rn(m1, dz1, g2z));
+                }
+            }
+        }
+        if (G) {
+            __syncwarp();
+            scatter_rows(f, k, gw + 3 * i, has2 ? gw + 3 * i2 : nullptr);
+            __syncwarp();
+        }
+    }
+    return acc;
+}
+
 // Energy (thread partial, not reduced) and -- if G -- per-warp gradient buffers.
 // pos4: smem float4-strided coordinates; gbuf: NW x nv.  IRTAB: the staged class
-// table holds 1/R* (see stage_molecule).
+// table holds 1/R* (see stage_molecule).  This body serves FP64.
 template <class R, class A, int NW, bool G, bool IRTAB = false>
 __device__ __forceinline__ A eval_terms(const Params &P, const MolV &m, const R *pos4, R *gbuf,
-                                        const MolSmem &ms, int nv) {
+                                        const MolSmem &ms, int nv, int forms = t32::kFused) {
+    if constexpr (sizeof(R) == 4) {
+        static_assert(IRTAB, "the FP32 evaluation reads 1/R* tables");
+        return eval_terms32<A, NW, G>(P, m, pos4, gbuf, ms, nv, forms);
+    } else {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int N = m.n;
     A acc = A(0);
@@ -496,7 +691,7 @@ __device__ __forceinline__ A eval_terms(const Params &P, const MolV &m, const R 
                 const int cj = ms.cls[j];
                 const float2 t1 = ms.tab[ci + cj], t2 = ms.tab[ck + cj];
                 const uint32_t w14 = p14[i * W + wb], w14b = jb >= jb2 ? p14[i2 * W + wb] : 0u;
-                R q1 = pair_charge<R>(ms, i, j), q2 = pair_charge<R>(ms, ik, j);
+                R q1 = qprod<R>(ms.qa[i], ms.qa[j]), q2 = qprod<R>(ms.qa[ik], ms.qa[j]);
                 if ((w14 >> lane) & 1u) q1 *= R(0.75);
                 if ((w14b >> lane) & 1u) q2 *= R(0.75);
                 R xj, yj, zj;
@@ -538,6 +733,7 @@ __device__ __forceinline__ A eval_terms(const Params &P, const MolV &m, const R 
         }
     }
     return acc;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -558,7 +754,6 @@ struct Opt {
     bool use64;        // line-search energies in FP64 (escalated)
     int *cls;
     double *qa;
-    float *qf;
     uint32_t *mask;
     float2 *tab;
     MolSmem ms;
@@ -579,8 +774,8 @@ struct Opt {
         xo = (R *)(sm + L.xo); dg = (R *)(sm + L.dg); hp = (R *)(sm + L.hp); hq = (R *)(sm + L.hq);
         pxi = (R *)(sm + L.pxi); pc = (R *)(sm + L.pc); pr = (R *)(sm + L.pr); gbuf = (R *)(sm + L.gbuf);
         cls = (int *)(sm + L.cls); qa = (double *)(sm + L.q); red = (A *)(sm + L.red);
-        qf = (float *)(sm + L.qf); mask = (uint32_t *)(sm + L.mask); tab = (float2 *)(sm + L.tab);
-        ms.cls = cls; ms.qa = qa; ms.qf = qf; ms.mask = mask; ms.tab = tab;
+        mask = (uint32_t *)(sm + L.mask); tab = (float2 *)(sm + L.tab);
+        ms.cls = cls; ms.qa = qa; ms.mask = mask; ms.tab = tab;
         rho_s = (A *)(sm + L.rho); alpha_s = (A *)(sm + L.alpha);
         if (MSM) mat = (R *)(sm + L.mat);
         else mat = (R *)p.gmat + (size_t)blockIdx.x * p.gslot;
@@ -597,27 +792,36 @@ struct Opt {
         block_reduce<NW, KS, KM, A>(s, mm, next_red());
     }
 
+    // Energy (block-reduced) and per-warp gradient buffers at pos4, in the instance's term
+    // precision.  The reduction's barrier also publishes the buffers to gradient_at().
+    __device__ __forceinline__ A evaluate(bool first) {
+        constexpr int kFirst = t32::kBondApart | t32::kTorsionApart | (LB && MSM && NC == 0 ? t32::kStrbendApart : 0);
+        A e[1] = {eval_terms<R, A, NW, true, sizeof(R) == 4>(P, m, pos4, gbuf, ms, nv, first ? kFirst : t32::kFused)}, z[1] = {A(0)};
+        reduce<1, 1>(e, z);
+        return e[0];
+    }
+
+    // Energy alone in the instance's term precision (the bits of evaluate()'s energy).
     __device__ __forceinline__ A energy() {
-        A e[1];
-        if (sizeof(R) == 4 && use64)
-            e[0] = (A)eval_terms<double, double, NW, false, sizeof(R) == 4>(P, m, pos4d, (double *)nullptr, ms, nv);
-        else
-            e[0] = eval_terms<R, A, NW, false, sizeof(R) == 4>(P, m, pos4, gbuf, ms, nv);
+        A e[1] = {eval_terms<R, A, NW, false, sizeof(R) == 4>(P, m, pos4, gbuf, ms, nv)}, z[1] = {A(0)};
+        reduce<1, 1>(e, z);
+        return e[0];
+    }
+
+    // Energy alone with FP64 terms at the same coordinates (the polished line search).
+    __device__ __forceinline__ A energy64() {
+        A e[1] = {(A)eval_terms<double, double, NW, false, sizeof(R) == 4>(P, m, pos4d, (double *)nullptr, ms, nv)};
         A z[1] = {A(0)};
         reduce<1, 1>(e, z);
         return e[0];
     }
 
-    // gradient at pos4 into dst (raw, unscaled); needs a preceding __syncthreads after pos4 writes
-    __device__ __forceinline__ void gradient(R *dst) {
-        eval_terms<R, A, NW, true, sizeof(R) == 4>(P, m, pos4, gbuf, ms, nv);
-        __syncthreads();
-        for (int k = threadIdx.x; k < n; k += NT) {
-            R s = R(0);
+    // Component k of the raw gradient of the last evaluate(): the buffers in warp order.
+    __device__ __forceinline__ R gradient_at(int k) const {
+        R s = R(0);
 #pragma unroll
-            for (int w = 0; w < NW; ++w) s += gbuf[(size_t)w * nv + k];
-            dst[k] = s;
-        }
+        for (int w = 0; w < NW; ++w) s += gbuf[(size_t)w * nv + k];
+        return s;
     }
 
     __device__ __forceinline__ void setpos(int k, R v) {
@@ -967,6 +1171,18 @@ struct Opt {
         }
     }
 
+    // restart from steepest descent: identity H / empty history, direction -g
+    __device__ __forceinline__ void restart(int &restarts, bool &fresh, bool &pending, int &hcount, int &hidx) {
+        ++restarts;
+        fresh = true;
+        pending = false;
+        hcount = 0;
+        hidx = 0;
+        reset_matrix();
+        for (int k = threadIdx.x; k < n; k += NT) dir[k] = -g[k];
+        __syncthreads();
+    }
+
     __device__ void run(int conf) {
         const int tid = threadIdx.x;
         const KConst &K = P.K;
@@ -982,186 +1198,131 @@ struct Opt {
             x[k] = v;
             setpos(k, v);
         }
-        stage_molecule<NT, sizeof(R) == 4>(P, m, cls, qa, qf, mask, tab);
+        stage_molecule<NT, sizeof(R) == 4>(P, m, cls, qa, (float *)pos4, mask, tab);
         ldh = MSM ? n : hld(n);
         // zero vector pads: the float4 pass reads columns up to hld(n)
         for (int k = n + tid; k < nv; k += NT) { g[k] = R(0); dg[k] = R(0); pxi[k] = R(0); pc[k] = R(0); }
         if (!LB) reset_matrix();
         __syncthreads();
 
-        // initial gradient and scale (header :435-454, tg.metal:115-122)
-        gradient(hp);
-        A gs_[2] = {A(0), A(0)}, gm_[1] = {A(0)};
-        for (int k = tid; k < n; k += NT) {
-            gs_[0] += (A)fabs(hp[k]);
-            gs_[1] += (A)(x[k] * x[k]);
-            A a = (A)fabs(hp[k]);
-            gm_[0] = a > gm_[0] ? a : gm_[0];
-        }
-        reduce<2, 1>(gs_, gm_);
+        // An accepted trial's gradient is the next iteration's, so a trial that will probably be
+        // accepted is evaluated with its gradient (1.36 times an energy alone) instead of twice.
+        // A dense run rejects nearly every full step for its first 50 to 200 iterations (its
+        // directions start from an identity H) and accepts 90 % and more of them later, so the
+        // first trial is taken for rejected -- energy alone -- when the last iteration's was, and
+        // the first two trials of a run are; every other trial comes with its gradient.  (Without
+        // the energy-alone trials: 5.47 ms below.)  There is one inlined copy of the combined
+        // evaluation, at the head of the loop; the initial point, the trials and a failed
+        // search's kept point all pass through it, which also ends most of the 128-register
+        // instances' spills (152 -> 0 B, dense).  B200, 5000 conformers of 18-150 atoms, 5 dense
+        // iterations: 5.68 -> 4.83 ms; 672 of 131-369 atoms, 8 L-BFGS iterations: 3.37 -> 2.39 ms;
+        // to convergence, 2000 drug-like conformers: 205 -> 170 ms, 400 large: 541 -> 439 ms.
+        enum { kInit, kTrial, kKeep };
+        int mode = kInit;
         R gsc = (R)K.gscale;
-        {
-            // bounded: a non-finite gradient is caught below, never halved forever
-            R mx = (R)gm_[0] * gsc;
-            for (int h = 0; h < 256 && mx > (R)K.gcap; ++h) { mx *= R(0.5); gsc *= R(0.5); }
-        }
-        for (int k = tid; k < n; k += NT) {
-            R v = hp[k] * gsc;
-            g[k] = v;
-            dir[k] = -v;
-        }
-        A E = energy();
-        const A max_step = (A)K.maxstep * (sqrt(gs_[1]) > (A)n ? sqrt(gs_[1]) : (A)n);
+        A E = A(0), max_step = A(0), slope = A(0), lam_min = A(0), Eold = A(0);
+        A lam = A(1), plam = A(1), pe = A(0);
         int status = MMFFB_ST_MAXIT;
-        int it = 0, done_iters = 0, nevals = 0, restarts = 0;
+        int it = 0, done_iters = 0, nevals = 0, restarts = 0, ls = 0;
+        int etrials = 2;       // trials of this iteration that are taken for rejected ones
         bool fresh = true;     // direction is -g (start or just after a restart)
         bool pending = false;  // a rank-2 update not yet applied to H
         int hcount = 0, hidx = 0;
-        if (!isfinite((double)E) || !isfinite((double)gs_[0])) {
-            status = MMFFB_ST_NONFINITE;
-            it = P.max_iters;
-        } else {
-            for (it = 0; it < P.max_iters; ++it) {
-                // direction length, slope, largest relative component; xold = x
-                A s3[2] = {A(0), A(0)}, m3[1] = {A(0)};
-                for (int k = tid; k < n; k += NT) {
-                    const R d = dir[k], xv = x[k];
-                    xo[k] = xv;
-                    s3[0] += (A)(d * d);
-                    s3[1] += (A)(d * g[k]);
-                    A t = (A)(fabs(d) / fmax(fabs(xv), R(1)));
-                    m3[0] = t > m3[0] ? t : m3[0];
+        for (;;) {
+            A et = A(0);
+            bool accept = true;
+            const bool energy_first = mode == kTrial && ((sizeof(R) == 4 && use64) || ls < etrials);
+            if (energy_first) {
+                et = sizeof(R) == 4 && use64 ? energy64() : energy();
+                accept = et - Eold <= (A)K.functol * lam * slope;
+            }
+            if (accept) {
+                const A e = evaluate(mode == kInit);
+                if (!energy_first) {
+                    et = e;
+                    if (mode == kTrial) accept = et - Eold <= (A)K.functol * lam * slope;
                 }
-                reduce<2, 1>(s3, m3);
-                const A dn = sqrt(s3[0]);
-                if (dn > max_step) {
-                    const R sc = (R)(max_step / dn);
-                    A s4[1] = {A(0)}, m4[1] = {A(0)};
-                    for (int k = tid; k < n; k += NT) {
-                        const R d = dir[k] * sc;
-                        dir[k] = d;
-                        s4[0] += (A)(d * g[k]);
-                        A t = (A)(fabs(d) / fmax(fabs(x[k]), R(1)));
-                        m4[0] = t > m4[0] ? t : m4[0];
-                    }
-                    reduce<1, 1>(s4, m4);
-                    s3[1] = s4[0];
-                    m3[0] = m4[0];
-                }
-                const A slope = s3[1];
-                if (!(slope < A(0))) {
-                    if (!fresh && restarts < P.max_restarts) {
-                        // uphill quasi-Newton direction: restart from steepest descent
-                        ++restarts;
-                        fresh = true;
-                        pending = false;
-                        hcount = 0;
-                        hidx = 0;
-                        reset_matrix();
-                        for (int k = tid; k < n; k += NT) dir[k] = -g[k];
-                        __syncthreads();
-                        continue;
-                    }
-                    status = MMFFB_ST_SLOPE;
-                    break;
-                }
-                const A lam_min = (A)K.movetol / (m3[0] > A(1e-30) ? m3[0] : A(1e-30));
-
-                // backtracking line search (tg.metal:192-256)
-                const A Eold = E;
-                A lam = A(1), plam = A(1), pe = Eold;
-                bool ok = false;
-                for (int ls = 0; ls < K.maxls; ++ls) {
-                    if (lam < lam_min) break;
-                    ++nevals;
-                    const R lr = (R)lam;
-                    for (int k = tid; k < n; k += NT) {
-                        const R v = xo[k] + lr * dir[k];
-                        x[k] = v;
-                        setpos(k, v);
-                    }
-                    __syncthreads();
-                    const A et = energy();
-                    if (et - Eold <= (A)K.functol * lam * slope) { E = et; ok = true; break; }
-                    A tl;
-                    if (ls == 0) {
-                        tl = -slope / (A(2) * (et - Eold - slope));
-                    } else {
-                        const A r1 = et - Eold - lam * slope, r2 = pe - Eold - plam * slope;
-                        const A l2 = lam * lam, p2 = plam * plam, dv = lam - plam;
-                        if (fabs(dv) < A(1e-30)) tl = A(0.5) * lam;
+            }
+            bool begin = accept;   // the next point opens a new iteration
+            if (!accept) {
+                // backtrack (tg.metal:192-256)
+                A tl;
+                if (ls == 0) {
+                    tl = -slope / (A(2) * (et - Eold - slope));
+                } else {
+                    const A r1 = et - Eold - lam * slope, r2 = pe - Eold - plam * slope;
+                    const A l2 = lam * lam, p2 = plam * plam, dv = lam - plam;
+                    if (fabs(dv) < A(1e-30)) tl = A(0.5) * lam;
+                    else {
+                        const A a = (r1 / l2 - r2 / p2) / dv, b = (-plam * r1 / l2 + lam * r2 / p2) / dv;
+                        if (fabs(a) < A(1e-30)) tl = fabs(b) > A(1e-30) ? -slope / (A(2) * b) : A(0.5) * lam;
                         else {
-                            const A a = (r1 / l2 - r2 / p2) / dv, b = (-plam * r1 / l2 + lam * r2 / p2) / dv;
-                            if (fabs(a) < A(1e-30)) tl = fabs(b) > A(1e-30) ? -slope / (A(2) * b) : A(0.5) * lam;
-                            else {
-                                const A disc = b * b - A(3) * a * slope;
-                                if (disc < A(0)) tl = A(0.5) * lam;
-                                else if (b <= A(0)) tl = (-b + sqrt(disc)) / (A(3) * a);
-                                else tl = -slope / (b + sqrt(disc));
-                            }
+                            const A disc = b * b - A(3) * a * slope;
+                            if (disc < A(0)) tl = A(0.5) * lam;
+                            else if (b <= A(0)) tl = (-b + sqrt(disc)) / (A(3) * a);
+                            else tl = -slope / (b + sqrt(disc));
                         }
                     }
-                    tl = tl < A(0.5) * lam ? tl : A(0.5) * lam;
-                    tl = tl > A(0.1) * lam ? tl : A(0.1) * lam;
-                    plam = lam; pe = et; lam = tl;
                 }
-                if (!ok) {
-                    for (int k = tid; k < n; k += NT) {
-                        x[k] = xo[k];
-                        setpos(k, xo[k]);
-                    }
-                    if (sizeof(R) == 4 && P.polish64 && !use64) {
-                        // FP32 term energies are at their noise floor: continue with FP64
-                        // line-search energies of the same FP32 coordinates
-                        use64 = true;
-                        __syncthreads();
-                        E = energy();
-                        continue;
-                    }
-                    if (!fresh && restarts < P.max_restarts) {
-                        // no decrease along the quasi-Newton direction: restart from -g
-                        ++restarts;
-                        fresh = true;
-                        pending = false;
-                        hcount = 0;
-                        hidx = 0;
-                        reset_matrix();
-                        for (int k = tid; k < n; k += NT) dir[k] = -g[k];
-                        __syncthreads();
-                        continue;
-                    }
-                    __syncthreads();
-                }
-                fresh = false;
-                // xi = x - xold, TOLX (kept per thread until the next reduction)
-                A tolx = A(0);
+                tl = tl < A(0.5) * lam ? tl : A(0.5) * lam;
+                tl = tl > A(0.1) * lam ? tl : A(0.1) * lam;
+                plam = lam; pe = et; lam = tl;
+                ++ls;
+            } else if (mode == kInit) {
+                // initial gradient and scale (header :435-454, tg.metal:115-122)
+                E = et;
+                A gs_[2] = {A(0), A(0)}, gm_[1] = {A(0)};
                 for (int k = tid; k < n; k += NT) {
-                    const R xi = x[k] - xo[k];
-                    xo[k] = xi;
-                    A t = (A)(fabs(xi) / fmax(fabs(x[k]), R(1)));
-                    tolx = t > tolx ? t : tolx;
+                    const R v = gradient_at(k);
+                    hp[k] = v;
+                    gs_[0] += (A)fabs(v);
+                    gs_[1] += (A)(x[k] * x[k]);
+                    A a = (A)fabs(v);
+                    gm_[0] = a > gm_[0] ? a : gm_[0];
                 }
-                // gradient at the new point (computed before the TOLX verdict; one
-                // wasted evaluation per conformer instead of a barrier per iteration)
-                gradient(hp);
+                reduce<2, 1>(gs_, gm_);
+                {
+                    // bounded: a non-finite gradient is caught below, never halved forever
+                    R mx = (R)gm_[0] * gsc;
+                    for (int h = 0; h < 256 && mx > (R)K.gcap; ++h) { mx *= R(0.5); gsc *= R(0.5); }
+                }
+                for (int k = tid; k < n; k += NT) {
+                    R v = hp[k] * gsc;
+                    g[k] = v;
+                    dir[k] = -v;
+                }
+                max_step = (A)K.maxstep * (sqrt(gs_[1]) > (A)n ? sqrt(gs_[1]) : (A)n);
+                if (!isfinite((double)E) || !isfinite((double)gs_[0])) {
+                    status = MMFFB_ST_NONFINITE;
+                    it = P.max_iters;
+                    break;
+                }
+            } else {
+                const bool ok = mode == kTrial;
+                if (ok) E = et;
+                etrials = ls > 0 ? 1 : 0;
+                fresh = false;
+                // xi = x - xold, TOLX, and the norms of the gradient at the new point
                 const bool atom_test = P.exit_test == MMFFB_EXIT_ATOM_NORM &&
                                        (P.check_every <= 1 || (it + 1) % P.check_every == 0);
-                A anorm = A(0);
+                A gs2[1] = {A(0)}, gm2[4] = {A(0), A(0), A(0), A(0)};
+                for (int k = tid; k < n; k += NT) {
+                    const R xv = x[k], xi = xv - xo[k], xm = fmax(fabs(xv), R(1)), gv = gradient_at(k);
+                    xo[k] = xi;
+                    hp[k] = gv;
+                    const A t = (A)(fabs(xi) / xm), a = (A)fabs(gv), b = (A)(fabs(gv) * xm);
+                    gs2[0] += a;
+                    gm2[0] = a > gm2[0] ? a : gm2[0];
+                    gm2[1] = b > gm2[1] ? b : gm2[1];
+                    gm2[2] = t > gm2[2] ? t : gm2[2];
+                }
                 if (atom_test) {
                     __syncthreads();
                     for (int a = tid; a < N; a += NT) {
                         const R gx = hp[3 * a], gy = hp[3 * a + 1], gz = hp[3 * a + 2];
                         const A v = (A)sqrt(gx * gx + gy * gy + gz * gz);
-                        anorm = v > anorm ? v : anorm;
+                        gm2[3] = v > gm2[3] ? v : gm2[3];
                     }
-                }
-                A gs2[1] = {A(0)}, gm2[4] = {A(0), A(0), tolx, anorm};
-                for (int k = tid; k < n; k += NT) {
-                    const A a = (A)fabs(hp[k]);
-                    gs2[0] += a;
-                    gm2[0] = a > gm2[0] ? a : gm2[0];
-                    const A b = (A)(fabs(hp[k]) * fmax(fabs(x[k]), R(1)));
-                    gm2[1] = b > gm2[1] ? b : gm2[1];
                 }
                 reduce<1, 4>(gs2, gm2);
                 if (!isfinite((double)gs2[0]) || !isfinite((double)E)) { status = MMFFB_ST_NONFINITE; break; }
@@ -1169,7 +1330,7 @@ struct Opt {
                 if (gm2[2] < (A)K.tolx) {
                     if (sizeof(R) == 4 && P.polish64 && !use64) {
                         use64 = true;
-                        E = energy();
+                        E = energy64();
                     } else {
                         status = ok ? MMFFB_ST_TOLX : MMFFB_ST_LSFAIL;
                         break;
@@ -1243,7 +1404,96 @@ struct Opt {
                     __syncthreads();
                     two_loop(hcount, hidx);
                 }
+                ++it;
             }
+            // the next point to evaluate
+            bool stop = false;
+            for (;;) {
+                if (begin) {
+                    if (it >= P.max_iters) { stop = true; break; }
+                    // direction length, slope, largest relative component; xold = x
+                    A s3[2] = {A(0), A(0)}, m3[1] = {A(0)};
+                    for (int k = tid; k < n; k += NT) {
+                        const R d = dir[k], xv = x[k];
+                        xo[k] = xv;
+                        s3[0] += (A)(d * d);
+                        s3[1] += (A)(d * g[k]);
+                        A t = (A)(fabs(d) / fmax(fabs(xv), R(1)));
+                        m3[0] = t > m3[0] ? t : m3[0];
+                    }
+                    reduce<2, 1>(s3, m3);
+                    const A dn = sqrt(s3[0]);
+                    if (dn > max_step) {
+                        const R sc = (R)(max_step / dn);
+                        A s4[1] = {A(0)}, m4[1] = {A(0)};
+                        for (int k = tid; k < n; k += NT) {
+                            const R d = dir[k] * sc;
+                            dir[k] = d;
+                            s4[0] += (A)(d * g[k]);
+                            A t = (A)(fabs(d) / fmax(fabs(x[k]), R(1)));
+                            m4[0] = t > m4[0] ? t : m4[0];
+                        }
+                        reduce<1, 1>(s4, m4);
+                        s3[1] = s4[0];
+                        m3[0] = m4[0];
+                    }
+                    slope = s3[1];
+                    if (!(slope < A(0))) {
+                        if (!fresh && restarts < P.max_restarts) {
+                            // uphill quasi-Newton direction: restart from steepest descent
+                            restart(restarts, fresh, pending, hcount, hidx);
+                            ++it;
+                            continue;
+                        }
+                        status = MMFFB_ST_SLOPE;
+                        stop = true;
+                        break;
+                    }
+                    lam_min = (A)K.movetol / (m3[0] > A(1e-30) ? m3[0] : A(1e-30));
+                    Eold = E;
+                    lam = plam = A(1);
+                    pe = Eold;
+                    ls = 0;
+                    begin = false;
+                }
+                if (ls < K.maxls && !(lam < lam_min)) {
+                    ++nevals;
+                    const R lr = (R)lam;
+                    for (int k = tid; k < n; k += NT) {
+                        const R v = xo[k] + lr * dir[k];
+                        x[k] = v;
+                        setpos(k, v);
+                    }
+                    mode = kTrial;
+                    break;
+                }
+                // no decrease along this direction: back to xold
+                for (int k = tid; k < n; k += NT) {
+                    x[k] = xo[k];
+                    setpos(k, xo[k]);
+                }
+                if (sizeof(R) == 4 && P.polish64 && !use64) {
+                    // FP32 term energies are at their noise floor: continue with FP64
+                    // line-search energies of the same FP32 coordinates
+                    use64 = true;
+                    __syncthreads();
+                    E = energy64();
+                    ++it;
+                    begin = true;
+                    continue;
+                }
+                if (!fresh && restarts < P.max_restarts) {
+                    // no decrease along the quasi-Newton direction: restart from -g
+                    restart(restarts, fresh, pending, hcount, hidx);
+                    ++it;
+                    begin = true;
+                    continue;
+                }
+                mode = kKeep;
+                break;
+            }
+            if (stop) break;
+            __syncthreads();
         }
         if (status != MMFFB_ST_NONFINITE || it < P.max_iters)
             done_iters = it < P.max_iters ? it + (status == MMFFB_ST_SLOPE ? 0 : 1) : P.max_iters;
@@ -1317,7 +1567,6 @@ __global__ void __launch_bounds__(NT) energy_grad_kernel(const Params P, float *
     R *pos4 = (R *)(smem + L.pos4), *gbuf = (R *)(smem + L.gbuf);
     int *cls = (int *)(smem + L.cls);
     double *qa = (double *)(smem + L.q);
-    float *qf = (float *)(smem + L.qf);
     uint32_t *mask = (uint32_t *)(smem + L.mask);
     float2 *tab = (float2 *)(smem + L.tab);
     A *red = (A *)(smem + L.red);
@@ -1325,8 +1574,8 @@ __global__ void __launch_bounds__(NT) energy_grad_kernel(const Params P, float *
     const int n = 3 * m.n, nv = (3 * P.nmax + 3) & ~3;
     const float *gp = P.pos + P.c.conf_coord[conf];
     for (int k = threadIdx.x; k < n; k += NT) pos4[4 * (k / 3) + (k % 3)] = (R)gp[k];
-    stage_molecule<NT, sizeof(R) == 4>(P, m, cls, qa, qf, mask, tab);
-    const MolSmem ms{cls, qa, qf, mask, tab};
+    stage_molecule<NT, sizeof(R) == 4>(P, m, cls, qa, (float *)pos4, mask, tab);
+    const MolSmem ms{cls, qa, mask, tab};
     __syncthreads();
     A e[1], z[1] = {A(0)};
     if (grad) e[0] = eval_terms<R, A, NW, true, sizeof(R) == 4>(P, m, pos4, gbuf, ms, nv);
@@ -1359,7 +1608,6 @@ __global__ void __launch_bounds__(NT) check64_kernel(const Params P, const doubl
     double *pos4 = (double *)(smem + L.pos4), *gbuf = (double *)(smem + L.gbuf);
     int *cls = (int *)(smem + L.cls);
     double *qa = (double *)(smem + L.q);
-    float *qf = (float *)(smem + L.qf);
     uint32_t *mask = (uint32_t *)(smem + L.mask);
     float2 *tab = (float2 *)(smem + L.tab);
     double *red = (double *)(smem + L.red);
@@ -1367,8 +1615,8 @@ __global__ void __launch_bounds__(NT) check64_kernel(const Params P, const doubl
     const int n = 3 * m.n, nv = (3 * P.nmax + 3) & ~3;
     const float *gp = P.pos + P.c.conf_coord[conf];
     for (int k = threadIdx.x; k < n; k += NT) pos4[4 * (k / 3) + (k % 3)] = (double)gp[k];
-    stage_molecule<NT, false>(P, m, cls, qa, qf, mask, tab);
-    const MolSmem ms{cls, qa, qf, mask, tab};
+    stage_molecule<NT, false>(P, m, cls, qa, nullptr, mask, tab);
+    const MolSmem ms{cls, qa, mask, tab};
     __syncthreads();
     double s[2], z[1] = {0.0};
     s[0] = eval_terms<double, double, NW, true, false>(P, m, pos4, gbuf, ms, nv);

@@ -48,7 +48,6 @@ __global__ void __launch_bounds__(NT) multimol_kernel(const MMArgs a) {
     float *qv = (float *)(smem + L.hq);
     int *cls = (int *)(smem + L.cls);
     double *qa = (double *)(smem + L.q);
-    float *qf = (float *)(smem + L.qf);
     uint32_t *mask = (uint32_t *)(smem + L.mask);
     float2 *tab = (float2 *)(smem + L.tab);
     double *red0 = (double *)(smem + L.red), *red1 = red0 + NW * 8;
@@ -63,8 +62,8 @@ __global__ void __launch_bounds__(NT) multimol_kernel(const MMArgs a) {
     float *X = a.S.x + off, *G = a.S.g + off, *BX = a.S.best_x + off;
     float *Sh = a.S.hist + (size_t)conf * 2 * a.hist_m * a.nv, *Yh = Sh + (size_t)a.hist_m * a.nv;
     float *rho = a.S.rho + (size_t)conf * a.hist_m;
-    stage_molecule<NT, true>(P, m, cls, qa, qf, mask, tab);
-    const MolSmem ms{cls, qa, qf, mask, tab};
+    stage_molecule<NT, true>(P, m, cls, qa, pos4, mask, tab);
+    const MolSmem ms{cls, qa, mask, tab};
 
     // energy and scaled gradient at xv (into e, gv)
     auto eval = [&](double &e) {

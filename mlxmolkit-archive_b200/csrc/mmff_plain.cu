@@ -325,7 +325,6 @@ __global__ void __launch_bounds__(NT) fused_sd_kernel(const Params P, float max_
     R *pp = (R *)(smem + L.xo), *pg = (R *)(smem + L.dg), *gbuf = (R *)(smem + L.gbuf);
     int *cls = (int *)(smem + L.cls);
     double *qa = (double *)(smem + L.q);
-    float *qf = (float *)(smem + L.qf);
     uint32_t *mask = (uint32_t *)(smem + L.mask);
     float2 *tab = (float2 *)(smem + L.tab);
     A *red = (A *)(smem + L.red);
@@ -338,13 +337,13 @@ __global__ void __launch_bounds__(NT) fused_sd_kernel(const Params P, float max_
         x[k] = v; pp[k] = v; pg[k] = R(0);
         pos4[4 * (k / 3) + (k % 3)] = v;
     }
-    stage_molecule<NT>(P, m, cls, qa, qf, mask, tab);
-    const MolSmem ms{cls, qa, qf, mask, tab};
+    stage_molecule<NT, true>(P, m, cls, qa, pos4, mask, tab);
+    const MolSmem ms{cls, qa, mask, tab};
     __syncthreads();
     R alpha = grad_lr;
     A E = A(0), Eprev = A(1e30);
     for (int it = 0; it < P.max_iters; ++it) {
-        A e1[1] = {eval_terms<R, A, NW, true>(P, m, pos4, gbuf, ms, nv)}, z[1] = {A(0)};
+        A e1[1] = {eval_terms<R, A, NW, true, true>(P, m, pos4, gbuf, ms, nv)}, z[1] = {A(0)};
         __syncthreads();
         for (int k = tid; k < n; k += NT) {
             R s = R(0);
