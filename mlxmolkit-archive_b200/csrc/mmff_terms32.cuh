@@ -20,6 +20,20 @@ namespace t32 {
 #define A_(a, b) __fadd_rn(a, b)
 #define F_(a, b, c) __fmaf_rn(a, b, c)
 
+// 1 / x and 1 / sqrt(x) of the hardware, for normal x: the bits of __fdividef(1, x) and
+// rsqrtf(x) without their steps for denormals (no argument below is one: each is bounded below
+// by 1e-30 or is a sum with a constant).
+__device__ __forceinline__ float rcp(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rsq(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 struct V3 {
     float x, y, z;
 };
@@ -38,7 +52,7 @@ __device__ __forceinline__ V3 subm(const V3 &a, float c, const V3 &b) {
     return V3{F_(-c, b.x, a.x), F_(-c, b.y, a.y), F_(-c, b.z, a.z)};
 }
 __device__ __forceinline__ float dot(const V3 &a, const V3 &b) { return F_(a.z, b.z, F_(a.x, b.x, M_(a.y, b.y))); }
-__device__ __forceinline__ float rinv(const V3 &a) { return rsqrtf(fmaxf(dot(a, a), 1e-16f)); }
+__device__ __forceinline__ float rinv(const V3 &a) { return rsq(fmaxf(dot(a, a), 1e-16f)); }
 __device__ __forceinline__ float clamp1(float c) { return c < -1.0f ? -1.0f : (c > 1.0f ? 1.0f : c); }
 __device__ __forceinline__ V3 cross(const V3 &a, const V3 &b) {
     return V3{F_(a.y, b.z, -M_(a.z, b.y)), F_(a.z, b.x, -M_(a.x, b.z)), F_(a.x, b.y, -M_(a.y, b.x))};
@@ -84,12 +98,12 @@ __device__ __forceinline__ float one_minus_sq(float c, bool apart) {
 template <bool G>
 __device__ __forceinline__ float bond(const V3 &a, const V3 &b, float kb, float r0, bool apart, V3 &f) {
     const V3 r = sub(a, b);
-    const float x2 = fmaxf(dot(r, r), 1e-16f), rs = rsqrtf(x2);
+    const float x2 = fmaxf(dot(r, r), 1e-16f), rs = rsq(x2);
     const float de = F_(x2, rs, -r0);
     const float ce = F_(M_(7.0f / 3.0f, de), de, F_(-2.0f, de, 1.0f));
     if (G) {
         const float d = M_(x2, rs), dr = apart ? A_(d, -r0) : de;
-        const float inv = d > 1e-8f ? __fdividef(1.0f, d) : 0.0f;
+        const float inv = d > 1e-8f ? rcp(d) : 0.0f;
         const float cg = F_(M_(14.0f / 3.0f, dr), dr, F_(-3.0f, dr, 1.0f));
         f = mul(M_(M_(M_(M_((float)MMFF_MDYNE, kb), dr), cg), inv), r);
     }
@@ -109,8 +123,8 @@ __device__ __forceinline__ float angle(const V3 &pi, const V3 &pj, const V3 &pk,
         const float sn2 = F_(-c, c, 1.0f);
         float cf = 0.0f;
         if (sn2 >= 1e-16f) {
-            const float rs = rsqrtf(fmaxf(sn2, 1e-16f)), sm = fmaxf(sn2, 0.0f);
-            const float de = linear ? M_(M_(-(float)MMFF_MDYNE, ka), M_(sm, rsqrtf(sm)))
+            const float rs = rsq(fmaxf(sn2, 1e-16f)), sm = fmaxf(sn2, 0.0f);
+            const float de = linear ? M_(M_(-(float)MMFF_MDYNE, ka), M_(sm, rsq(sm)))
                                     : M_(M_(M_(md.kang_deg, ka), dt), F_(md.cb15, dt, 1.0f));
             cf = M_(-de, rs);
         }
@@ -132,7 +146,7 @@ __device__ __forceinline__ float strbend(const V3 &pi, const V3 &pj, const V3 &p
     const V3 r1 = sub(pi, pj), r2 = sub(pk, pj);
     const float id1 = rinv(r1), id2 = rinv(r2);
     const float c = clamp1(M_(M_(dot(r1, r2), id1), id2));
-    const float d1 = __fdividef(1.0f, fmaxf(id1, 1e-8f)), d2 = __fdividef(1.0f, fmaxf(id2, 1e-8f));
+    const float d1 = rcp(fmaxf(id1, 1e-8f)), d2 = rcp(fmaxf(id2, 1e-8f));
     const float dt = F_((float)MMFF_RAD2DEG, acosf(c), -t0);
     const float dr1 = A_(d1, -r0ij), dr2 = A_(d2, -r0kj);
     const float ks = F_(dr1, kij, M_(dr2, kkj));
@@ -140,7 +154,7 @@ __device__ __forceinline__ float strbend(const V3 &pi, const V3 &pj, const V3 &p
         const float sn2 = one_minus_sq(c, apart);
         f0 = f1 = f2 = V3{0.0f, 0.0f, 0.0f};
         if (sn2 >= 1e-16f) {
-            const float is = fminf(rsqrtf(fmaxf(sn2, 1e-16f)), 1e8f), pf = md.ksbg;
+            const float is = fminf(rsq(fmaxf(sn2, 1e-16f)), 1e8f), pf = md.ksbg;
             const float beis = M_(M_((float)MMFF_RAD2DEG, ks), is);
             const V3 u1 = mul(id1, r1), u2 = mul(id2, r2);
             const V3 i1 = mul(id1, subm(u2, c, u1)), i3 = mul(id2, subm(u1, c, u2));
@@ -169,9 +183,9 @@ __device__ __forceinline__ float oop(const V3 &pi, const V3 &pj, const V3 &pk, c
     const float chi = M_((float)MMFF_RAD2DEG, asinf(s));
     if (G) {
         const float c2 = F_(-s, s, 1.0f);
-        const float ic = c2 > 0.0f ? rsqrtf(fmaxf(c2, 1e-16f)) : 1e8f;
+        const float ic = c2 > 0.0f ? rsq(fmaxf(c2, 1e-16f)) : 1e8f;
         const float ct = clamp1(dot(uI, uK));
-        const float ist = rsqrtf(fmaxf(F_(-ct, ct, 1.0f), 1e-8f));
+        const float ist = rsq(fmaxf(F_(-ct, ct, 1.0f), 1e-8f));
         const float dE = M_(M_(md.kang_deg, koop), chi);
         const float t1 = M_(ic, ist), t2 = M_(M_(M_(s, ic), ist), ist);
         const V3 a1 = cross(uL, uK), a2 = cross(uI, uL), a3 = cross(uK, uI);
@@ -197,14 +211,14 @@ __device__ __forceinline__ float torsion(const V3 &p1, const V3 &p2, const V3 &p
     const float n1 = dot(c1, c1), n2 = dot(c2, c2), comb = M_(n1, n2);
     float e = 0.0f;
     if (comb >= 1e-16f) {
-        const float cp = clamp1(M_(dot(c1, c2), rsqrtf(comb)));
+        const float cp = clamp1(M_(dot(c1, c2), rsq(comb)));
         const float cos2 = F_(M_(2.0f, cp), cp, -1.0f), cos31 = F_(cp, F_(M_(4.0f, cp), cp, -3.0f), 1.0f);
         e = M_(0.5f, F_(V3_, cos31, F_(V1, A_(1.0f, cp), M_(V2, A_(1.0f, -cos2)))));
     }
     if (G) {
         f0 = f1 = f2 = f3 = V3{0.0f, 0.0f, 0.0f};
         if (n1 >= 1e-30f && n2 >= 1e-30f) {
-            const float i1 = fminf(rsqrtf(n1), 1e5f), i2 = fminf(rsqrtf(n2), 1e5f);
+            const float i1 = fminf(rsq(n1), 1e5f), i2 = fminf(rsq(n2), 1e5f);
             const V3 u1 = mul(i1, c1), u2 = mul(i2, c2);
             const float cp = clamp1(dot(u1, u2));
             const float sp2 = one_minus_sq(cp, apart);
@@ -229,23 +243,24 @@ __device__ __forceinline__ float torsion(const V3 &p1, const V3 &p2, const V3 &p
 }
 
 // ---- buffered 14-7 vdW and Coulomb of one pair; iR = 1 / R*; s: grad_i = s (p_i - p_j) ----
-template <bool G>
-__device__ __forceinline__ void pair(float dx, float dy, float dz, float iR, float eps, float qq, bool dd,
-                                     float &e_vdw, float &e_ele, float &s) {
+// DD: distance-dependent dielectric
+template <bool G, bool DD>
+__device__ __forceinline__ void pair(float dx, float dy, float dz, float iR, float eps, float qq, float &e_vdw,
+                                     float &e_ele, float &s) {
     const float x2 = fmaxf(F_(dz, dz, F_(dx, dx, M_(dy, dy))), 1e-16f);
-    const float rd = rsqrtf(x2), d = M_(x2, rd);
+    const float rd = rsq(x2), d = M_(x2, rd);
     const float q = M_(d, iR), q2 = M_(q, q), q6 = M_(M_(q2, q2), q2);
-    const float ib = __fdividef(1.0f, A_(q, 0.07f));
+    const float ib = rcp(A_(q, 0.07f));
     const float t = M_(1.07f, ib), t2 = M_(t, t), t7 = M_(M_(M_(t2, t2), t2), t);
-    const float iq = __fdividef(1.0f, fmaxf(F_(q6, q, 0.12f), 1e-30f));
+    const float iq = rcp(F_(q6, q, 0.12f));
     e_vdw = M_(M_(eps, t7), F_(1.12f, iq, -2.0f));
-    const float idp = __fdividef(1.0f, A_(d, 0.05f));
-    const float cq = M_((float)MMFF_ELEC, qq), ce = M_(cq, idp);
-    e_ele = dd ? M_(ce, idp) : ce;
+    const float idp = rcp(A_(d, 0.05f));
+    const float cq = M_((float)MMFF_ELEC, qq);
+    e_ele = DD ? M_(M_(cq, idp), idp) : M_(cq, idp);
     if (G) {
         const float inv = d > 1e-8f ? rd : 0.0f;
         const float br = F_(F_(-7.84f, iq, 14.0f), ib, M_(M_(M_(-7.84f, q6), iq), iq));
-        const float de = dd ? M_(M_(M_(M_(-2.0f, cq), idp), idp), idp) : M_(M_(-cq, idp), idp);
+        const float de = DD ? M_(M_(M_(M_(-2.0f, cq), idp), idp), idp) : M_(M_(-cq, idp), idp);
         s = M_(F_(M_(M_(eps, iR), t7), br, de), inv);
     }
 }
