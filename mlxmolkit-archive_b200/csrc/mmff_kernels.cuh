@@ -276,37 +276,68 @@ template <class T> __device__ __forceinline__ T wmax(T v) {
     return v;
 }
 
-// Block reduction of KS sums and KM maxima; every thread receives the results.
-// One __syncthreads: the caller alternates between two scratch halves.
-template <int NW, int KS, int KM, class A>
-__device__ __forceinline__ void block_reduce(A (&s)[KS], A (&m)[KM], A *red) {
+// Block reduction of KS sums (type A) and KM maxima (type M); every thread receives the results,
+// the same bits in all of them.  One __syncthreads: the caller alternates between two scratch
+// halves.  The warps' partial values are summed by lane groups of NW (a tree), so a thread reads
+// one partial value per 32 / NW results instead of NW per result.  What bounds it is latency: at
+// 256 threads about 10 dependent shuffle-and-add steps and the barrier.
+template <int NW, int KS, int KM, class A, class M>
+__device__ __forceinline__ void block_reduce(A (&s)[KS], M (&m)[KM > 0 ? KM : 1], A *red) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int VR = 32 / NW;    // results per round of the second stage
+    const int w = lane % NW, kv = lane / NW;
+    M *redm = reinterpret_cast<M *>(red + NW * KS);
 #pragma unroll
     for (int k = 0; k < KS; ++k) s[k] = wsum(s[k]);
 #pragma unroll
     for (int k = 0; k < KM; ++k) m[k] = wmax(m[k]);
-    constexpr int K = KS + KM;
     if (lane == 0) {
 #pragma unroll
-        for (int k = 0; k < KS; ++k) red[warp * K + k] = s[k];
+        for (int k = 0; k < KS; ++k) red[k * NW + warp] = s[k];
 #pragma unroll
-        for (int k = 0; k < KM; ++k) red[warp * K + KS + k] = m[k];
+        for (int k = 0; k < KM; ++k) redm[k * NW + warp] = m[k];
     }
     __syncthreads();
+    if constexpr (KS == 1) {
+        A v = red[w];
 #pragma unroll
-    for (int k = 0; k < KS; ++k) {
-        A t = A(0);
+        for (int o = NW / 2; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        s[0] = v;
+    } else {
 #pragma unroll
-        for (int w = 0; w < NW; ++w) t += red[w * K + k];
-        s[k] = t;
+        for (int r = 0; r < KS; r += VR) {
+            A v = r + kv < KS ? red[(r + kv) * NW + w] : A(0);
+#pragma unroll
+            for (int o = NW / 2; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+#pragma unroll
+            for (int k = 0; k < VR; ++k)
+                if (r + k < KS) s[r + k] = __shfl_sync(0xffffffffu, v, k * NW);
+        }
     }
+    if constexpr (KM == 1) {
+        M v = redm[w];
 #pragma unroll
-    for (int k = 0; k < KM; ++k) {
-        A t = red[KS + k];
+        for (int o = NW / 2; o; o >>= 1) { const M u = __shfl_xor_sync(0xffffffffu, v, o); v = u > v ? u : v; }
+        m[0] = v;
+    } else if constexpr (KM > 1) {
 #pragma unroll
-        for (int w = 1; w < NW; ++w) { A u = red[w * K + KS + k]; t = u > t ? u : t; }
-        m[k] = t;
+        for (int r = 0; r < KM; r += VR) {
+            M v = redm[(r + kv < KM ? r + kv : r) * NW + w];
+#pragma unroll
+            for (int o = NW / 2; o; o >>= 1) { const M u = __shfl_xor_sync(0xffffffffu, v, o); v = u > v ? u : v; }
+#pragma unroll
+            for (int k = 0; k < VR; ++k)
+                if (r + k < KM) m[r + k] = __shfl_sync(0xffffffffu, v, k * NW);
+        }
     }
+}
+
+// Block sum of one value.
+template <int NW, class A>
+__device__ __forceinline__ A block_sum(A v, A *red) {
+    A s[1] = {v}, none[1];
+    block_reduce<NW, 1, 0, A, A>(s, none, red);
+    return s[0];
 }
 
 template <class R> __device__ __forceinline__ void add3(R *dst, const R *f) {
@@ -800,32 +831,31 @@ struct Opt {
     }
 
     template <int KS, int KM>
-    __device__ __forceinline__ void reduce(A (&s)[KS], A (&mm)[KM]) {
-        block_reduce<NW, KS, KM, A>(s, mm, next_red());
+    __device__ __forceinline__ void reduce(A (&s)[KS], R (&mm)[KM]) {
+        block_reduce<NW, KS, KM, A, R>(s, mm, next_red());
     }
+    template <int KS>
+    __device__ __forceinline__ void reduce(A (&s)[KS]) {
+        A none[1];
+        block_reduce<NW, KS, 0, A, A>(s, none, next_red());
+    }
+    __device__ __forceinline__ A sum(A v) { return block_sum<NW, A>(v, next_red()); }
 
     // Energy (block-reduced) and per-warp gradient buffers at pos4, in the instance's term
     // precision.  The reduction's barrier also publishes the buffers to gradient_at().
     __device__ __forceinline__ A evaluate(bool first) {
         constexpr int kFirst = t32::kBondApart | t32::kTorsionApart | (LB && MSM && NC == 0 ? t32::kStrbendApart : 0);
-        A e[1] = {eval_terms<R, A, NW, true, sizeof(R) == 4>(P, m, pos4, gbuf, ms, nv, first ? kFirst : t32::kFused)}, z[1] = {A(0)};
-        reduce<1, 1>(e, z);
-        return e[0];
+        return sum(eval_terms<R, A, NW, true, sizeof(R) == 4>(P, m, pos4, gbuf, ms, nv, first ? kFirst : t32::kFused));
     }
 
     // Energy alone in the instance's term precision (the bits of evaluate()'s energy).
     __device__ __forceinline__ A energy() {
-        A e[1] = {eval_terms<R, A, NW, false, sizeof(R) == 4>(P, m, pos4, gbuf, ms, nv)}, z[1] = {A(0)};
-        reduce<1, 1>(e, z);
-        return e[0];
+        return sum(eval_terms<R, A, NW, false, sizeof(R) == 4>(P, m, pos4, gbuf, ms, nv));
     }
 
     // Energy alone with FP64 terms at the same coordinates (the polished line search).
     __device__ __forceinline__ A energy64() {
-        A e[1] = {(A)eval_terms<double, double, NW, false, sizeof(R) == 4>(P, m, pos4d, (double *)nullptr, ms, nv)};
-        A z[1] = {A(0)};
-        reduce<1, 1>(e, z);
-        return e[0];
+        return sum((A)eval_terms<double, double, NW, false, sizeof(R) == 4>(P, m, pos4d, (double *)nullptr, ms, nv));
     }
 
     // Component k of the raw gradient of the last evaluate(): the buffers in warp order.
@@ -1130,46 +1160,76 @@ struct Opt {
         fence_proxy_async_global();
     }
 
-    // L-BFGS two-loop recursion (lbfgs_tg.metal:264-292): dir = -H g from the ring history
+    // L-BFGS two-loop recursion (lbfgs_tg.metal:264-292): dir = -H g from the ring history.  Each
+    // of its 2 hcount steps is a block-wide dot product and an update of q that the next dot product
+    // follows from, so it is bound by the latency of the reductions (one barrier each): a step's
+    // update and the next step's products are one pass over the thread's own elements, and the
+    // scaling's two sums ride with the first dot product.  Measured with the
+    // one-stage tree of block_reduce on B200, 672 conformers of 131-369 atoms x 8 iterations: 2.15 ->
+    // 1.96 ms (300 of 131-170 atoms x 200: 13.1 -> 10.8 ms).
     __device__ __forceinline__ void two_loop(int hcount, int hidx) {
-        const int hm = P.hist_m;
+        const int hm = P.hist_m, tid = threadIdx.x;
         R *S = mat, *Y = mat + (size_t)hm * nv;
-        for (int k = threadIdx.x; k < n; k += NT) hq[k] = g[k];
-        for (int jj = hcount - 1; jj >= 0; --jj) {
-            int slot = ((hidx - 1 - (hcount - 1 - jj)) % hm + hm) % hm;
-            const R *Sj = S + (size_t)slot * nv;
-            A s1[1] = {A(0)}, z[1] = {A(0)};
-            for (int k = threadIdx.x; k < n; k += NT) s1[0] += (A)(Sj[k] * hq[k]);
-            reduce<1, 1>(s1, z);
-            A aj = rho_s[slot] * s1[0];
-            if (threadIdx.x == 0) alpha_s[jj] = aj;
-            const R *Yj = Y + (size_t)slot * nv;
-            const R ar = (R)aj;
-            for (int k = threadIdx.x; k < n; k += NT) hq[k] -= ar * Yj[k];
+        if (hcount == 0) {
+            for (int k = tid; k < n; k += NT) dir[k] = -g[k];
+            return;
         }
-        if (hcount > 0) {
-            int nw = ((hidx - 1) % hm + hm) % hm;
-            const R *Sn = S + (size_t)nw * nv, *Yn = Y + (size_t)nw * nv;
-            A s2[2] = {A(0), A(0)}, z[1] = {A(0)};
-            for (int k = threadIdx.x; k < n; k += NT) {
-                s2[0] += (A)(Sn[k] * Yn[k]);
-                s2[1] += (A)(Yn[k] * Yn[k]);
+        int slot = (hidx - 1) % hm;   // newest pair
+        const R *Sj = S + (size_t)slot * nv, *Yj = Y + (size_t)slot * nv;
+        A s3[3] = {A(0), A(0), A(0)};
+        for (int k = tid; k < n; k += NT) {
+            const R gk = g[k], sk = Sj[k], yk = Yj[k];
+            s3[0] += (A)(sk * gk);
+            s3[1] += (A)(sk * yk);
+            s3[2] += (A)(yk * yk);
+        }
+        reduce<3>(s3);
+        const R gam = (R)(s3[1] / (s3[2] > A(1e-30) ? s3[2] : A(1e-30)));
+        A dot = s3[0];
+        const R *q = g;               // q before this step's update
+        for (int jj = hcount - 1; jj >= 0; --jj) {
+            const A aj = rho_s[slot] * dot;
+            if (tid == 0) alpha_s[jj] = aj;
+            const R ar = (R)aj;
+            A part = A(0);
+            if (jj > 0) {
+                slot = slot > 0 ? slot - 1 : hm - 1;
+                const R *Sn = S + (size_t)slot * nv;
+                for (int k = tid; k < n; k += NT) {
+                    const R v = fma(-ar, Yj[k], q[k]);
+                    hq[k] = v;
+                    part += (A)(Sn[k] * v);
+                }
+                Yj = Y + (size_t)slot * nv;
+            } else {
+                // the oldest pair's update, the scaling, and the second loop's first product
+                for (int k = tid; k < n; k += NT) {
+                    const R yk = Yj[k], v = fma(-ar, yk, q[k]) * gam;
+                    hq[k] = v;
+                    part += (A)(yk * v);
+                }
             }
-            reduce<2, 1>(s2, z);
-            const R gam = (R)(s2[0] / (s2[1] > A(1e-30) ? s2[1] : A(1e-30)));
-            for (int k = threadIdx.x; k < n; k += NT) hq[k] *= gam;
+            q = hq;
+            dot = sum(part);
         }
         for (int jj = 0; jj < hcount; ++jj) {
-            int slot = ((hidx - 1 - (hcount - 1 - jj)) % hm + hm) % hm;
-            const R *Yj = Y + (size_t)slot * nv, *Sj = S + (size_t)slot * nv;
-            A s1[1] = {A(0)}, z[1] = {A(0)};
-            for (int k = threadIdx.x; k < n; k += NT) s1[0] += (A)(Yj[k] * hq[k]);
-            reduce<1, 1>(s1, z);
-            const A bj = rho_s[slot] * s1[0];
+            const A bj = rho_s[slot] * dot;
             const R c = (R)(alpha_s[jj] - bj);
-            for (int k = threadIdx.x; k < n; k += NT) hq[k] += c * Sj[k];
+            const R *So = S + (size_t)slot * nv;
+            if (jj + 1 < hcount) {
+                slot = slot + 1 < hm ? slot + 1 : 0;
+                const R *Yn = Y + (size_t)slot * nv;
+                A part = A(0);
+                for (int k = tid; k < n; k += NT) {
+                    const R v = fma(c, So[k], hq[k]);
+                    hq[k] = v;
+                    part += (A)(Yn[k] * v);
+                }
+                dot = sum(part);
+            } else {
+                for (int k = tid; k < n; k += NT) dir[k] = -fma(c, So[k], hq[k]);
+            }
         }
-        for (int k = threadIdx.x; k < n; k += NT) dir[k] = -hq[k];
     }
 
     // inverse Hessian back to the identity (dense) / history cleared (L-BFGS)
@@ -1283,19 +1343,20 @@ struct Opt {
             } else if (mode == kInit) {
                 // initial gradient and scale (header :435-454, tg.metal:115-122)
                 E = et;
-                A gs_[2] = {A(0), A(0)}, gm_[1] = {A(0)};
+                A gs_[2] = {A(0), A(0)};
+                R gm_[1] = {R(0)};
                 for (int k = tid; k < n; k += NT) {
                     const R v = gradient_at(k);
                     hp[k] = v;
                     gs_[0] += (A)fabs(v);
                     gs_[1] += (A)(x[k] * x[k]);
-                    A a = (A)fabs(v);
+                    const R a = fabs(v);
                     gm_[0] = a > gm_[0] ? a : gm_[0];
                 }
                 reduce<2, 1>(gs_, gm_);
                 {
                     // bounded: a non-finite gradient is caught below, never halved forever
-                    R mx = (R)gm_[0] * gsc;
+                    R mx = gm_[0] * gsc;
                     for (int h = 0; h < 256 && mx > (R)K.gcap; ++h) { mx *= R(0.5); gsc *= R(0.5); }
                 }
                 for (int k = tid; k < n; k += NT) {
@@ -1317,13 +1378,14 @@ struct Opt {
                 // xi = x - xold, TOLX, and the norms of the gradient at the new point
                 const bool atom_test = P.exit_test == MMFFB_EXIT_ATOM_NORM &&
                                        (P.check_every <= 1 || (it + 1) % P.check_every == 0);
-                A gs2[1] = {A(0)}, gm2[4] = {A(0), A(0), A(0), A(0)};
+                A gs2[1] = {A(0)};
+                R gm2[4] = {R(0), R(0), R(0), R(0)};
                 for (int k = tid; k < n; k += NT) {
                     const R xv = x[k], xi = xv - xo[k], xm = fmax(fabs(xv), R(1)), gv = gradient_at(k);
                     xo[k] = xi;
                     hp[k] = gv;
-                    const A t = (A)(fabs(xi) / xm), a = (A)fabs(gv), b = (A)(fabs(gv) * xm);
-                    gs2[0] += a;
+                    const R t = fabs(xi) / xm, a = fabs(gv), b = a * xm;
+                    gs2[0] += (A)a;
                     gm2[0] = a > gm2[0] ? a : gm2[0];
                     gm2[1] = b > gm2[1] ? b : gm2[1];
                     gm2[2] = t > gm2[2] ? t : gm2[2];
@@ -1332,14 +1394,14 @@ struct Opt {
                     __syncthreads();
                     for (int a = tid; a < N; a += NT) {
                         const R gx = hp[3 * a], gy = hp[3 * a + 1], gz = hp[3 * a + 2];
-                        const A v = (A)sqrt(gx * gx + gy * gy + gz * gz);
+                        const R v = sqrt(gx * gx + gy * gy + gz * gz);
                         gm2[3] = v > gm2[3] ? v : gm2[3];
                     }
                 }
                 reduce<1, 4>(gs2, gm2);
                 if (!isfinite((double)gs2[0]) || !isfinite((double)E)) { status = MMFFB_ST_NONFINITE; break; }
-                if (atom_test && gm2[3] * (A)P.atom_grad_scale <= (A)P.grad_tol) { status = MMFFB_ST_GRAD; break; }
-                if (gm2[2] < (A)K.tolx) {
+                if (atom_test && (A)gm2[3] * (A)P.atom_grad_scale <= (A)P.grad_tol) { status = MMFFB_ST_GRAD; break; }
+                if ((A)gm2[2] < (A)K.tolx) {
                     if (sizeof(R) == 4 && P.polish64 && !use64) {
                         use64 = true;
                         E = energy64();
@@ -1349,11 +1411,11 @@ struct Opt {
                     }
                 }
                 {
-                    R mx = (R)gm2[0] * gsc;
+                    R mx = gm2[0] * gsc;
                     for (int h = 0; h < 256 && mx > (R)K.gcap; ++h) { mx *= R(0.5); gsc *= R(0.5); }
                 }
                 if (P.exit_test == MMFFB_EXIT_TG) {
-                    const A num = (A)((R)gm2[1] * gsc);
+                    const A num = (A)(gm2[1] * gsc);
                     A den = E * (A)gsc;
                     den = den > A(1) ? den : A(1);
                     if (num / den < (A)P.grad_tol) { status = MMFFB_ST_GRAD; break; }
@@ -1370,7 +1432,7 @@ struct Opt {
                     else hpass_stream(pending);
                     __syncthreads();
                     if (!MSM && *(volatile int *)abort_flag) { status = MMFFB_ST_TIMEOUT; break; }
-                    A d6[6] = {A(0), A(0), A(0), A(0), A(0), A(0)}, z[1] = {A(0)};
+                    A d6[6] = {A(0), A(0), A(0), A(0), A(0), A(0)};
                     for (int k = tid; k < n; k += NT) {
                         const R dgk = dg[k], xik = xo[k], qk = hq[k], gk = g[k];
                         d6[0] += (A)(dgk * xik);
@@ -1380,7 +1442,7 @@ struct Opt {
                         d6[4] += (A)(xik * gk);
                         d6[5] += (A)(qk * gk);
                     }
-                    reduce<6, 1>(d6, z);
+                    reduce<6>(d6);
                     const A fac = d6[0], fae = d6[1];
                     if (fac * fac > (A)K.eps * d6[2] * d6[3] && fac > A(0)) {
                         const A fi = A(1) / fac;
@@ -1401,19 +1463,19 @@ struct Opt {
                     }
                 } else {
                     // L-BFGS history update (lbfgs_tg.metal:247-262)
-                    A y1[1] = {A(0)}, z[1] = {A(0)};
-                    for (int k = tid; k < n; k += NT) y1[0] += (A)(dg[k] * xo[k]);
-                    reduce<1, 1>(y1, z);
-                    if (y1[0] > A(1e-10)) {
+                    A y1 = A(0);
+                    for (int k = tid; k < n; k += NT) y1 += (A)(dg[k] * xo[k]);
+                    y1 = sum(y1);
+                    if (y1 > A(1e-10)) {
                         const int hm = P.hist_m;
                         const int slot = hidx % hm;
                         R *S = mat + (size_t)slot * nv, *Y = mat + (size_t)hm * nv + (size_t)slot * nv;
                         for (int k = tid; k < n; k += NT) { S[k] = xo[k]; Y[k] = dg[k]; }
-                        if (tid == 0) rho_s[slot] = A(1) / y1[0];
+                        if (tid == 0) rho_s[slot] = A(1) / y1;
                         hidx++;
                         if (hcount < hm) hcount++;
                     }
-                    __syncthreads();
+                    // each thread reads back its own elements only; rho is read after a barrier
                     two_loop(hcount, hidx);
                 }
                 ++it;
@@ -1424,25 +1486,27 @@ struct Opt {
                 if (begin) {
                     if (it >= P.max_iters) { stop = true; break; }
                     // direction length, slope, largest relative component; xold = x
-                    A s3[2] = {A(0), A(0)}, m3[1] = {A(0)};
+                    A s3[2] = {A(0), A(0)};
+                    R m3[1] = {R(0)};
                     for (int k = tid; k < n; k += NT) {
                         const R d = dir[k], xv = x[k];
                         xo[k] = xv;
                         s3[0] += (A)(d * d);
                         s3[1] += (A)(d * g[k]);
-                        A t = (A)(fabs(d) / fmax(fabs(xv), R(1)));
+                        const R t = fabs(d) / fmax(fabs(xv), R(1));
                         m3[0] = t > m3[0] ? t : m3[0];
                     }
                     reduce<2, 1>(s3, m3);
                     const A dn = sqrt(s3[0]);
                     if (dn > max_step) {
                         const R sc = (R)(max_step / dn);
-                        A s4[1] = {A(0)}, m4[1] = {A(0)};
+                        A s4[1] = {A(0)};
+                        R m4[1] = {R(0)};
                         for (int k = tid; k < n; k += NT) {
                             const R d = dir[k] * sc;
                             dir[k] = d;
                             s4[0] += (A)(d * g[k]);
-                            A t = (A)(fabs(d) / fmax(fabs(x[k]), R(1)));
+                            const R t = fabs(d) / fmax(fabs(x[k]), R(1));
                             m4[0] = t > m4[0] ? t : m4[0];
                         }
                         reduce<1, 1>(s4, m4);
@@ -1461,7 +1525,7 @@ struct Opt {
                         stop = true;
                         break;
                     }
-                    lam_min = (A)K.movetol / (m3[0] > A(1e-30) ? m3[0] : A(1e-30));
+                    lam_min = (A)K.movetol / ((A)m3[0] > A(1e-30) ? (A)m3[0] : A(1e-30));
                     Eold = E;
                     lam = plam = A(1);
                     pe = Eold;
@@ -1589,10 +1653,10 @@ __global__ void __launch_bounds__(NT) energy_grad_kernel(const Params P, float *
     stage_molecule<NT, sizeof(R) == 4>(P, m, cls, qa, (float *)pos4, mask, tab);
     const MolSmem ms{cls, qa, mask, tab};
     __syncthreads();
-    A e[1], z[1] = {A(0)};
+    A e[1];
     if (grad) e[0] = eval_terms<R, A, NW, true, sizeof(R) == 4>(P, m, pos4, gbuf, ms, nv);
     else e[0] = eval_terms<R, A, NW, false, sizeof(R) == 4>(P, m, pos4, gbuf, ms, nv);
-    block_reduce<NW, 1, 1, A>(e, z, red);
+    e[0] = block_sum<NW, A>(e[0], red);
     if (grad) {
         float *go = grad + P.c.conf_coord[conf];
         for (int k = threadIdx.x; k < n; k += NT) {
@@ -1630,7 +1694,7 @@ __global__ void __launch_bounds__(NT) check64_kernel(const Params P, const doubl
     stage_molecule<NT, false>(P, m, cls, qa, nullptr, mask, tab);
     const MolSmem ms{cls, qa, mask, tab};
     __syncthreads();
-    double s[2], z[1] = {0.0};
+    double s[2], none[1];
     s[0] = eval_terms<double, double, NW, true, false>(P, m, pos4, gbuf, ms, nv);
     __syncthreads();
     s[1] = 0.0;
@@ -1640,7 +1704,7 @@ __global__ void __launch_bounds__(NT) check64_kernel(const Params P, const doubl
         for (int w = 0; w < NW; ++w) g += gbuf[(size_t)w * nv + k];
         s[1] += g * g;
     }
-    block_reduce<NW, 2, 1, double>(s, z, red);
+    block_reduce<NW, 2, 0, double, double>(s, none, red);
     if (threadIdx.x == 0) {
         e64[conf] = s[0];
         if (derr) derr[conf] = e_in[conf] - s[0];

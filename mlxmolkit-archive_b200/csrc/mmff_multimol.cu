@@ -30,13 +30,6 @@ struct MMArgs {
     int nv;                    // history row stride
 };
 
-template <int NW>
-__device__ __forceinline__ double block_sum(double v, double *red) {
-    double s[1] = {v}, z[1] = {0.0};
-    block_reduce<NW, 1, 1, double>(s, z, red);
-    return s[0];
-}
-
 template <int NT>
 __global__ void __launch_bounds__(NT) multimol_kernel(const MMArgs a) {
     constexpr int NW = NT / 32;
@@ -77,7 +70,7 @@ __global__ void __launch_bounds__(NT) multimol_kernel(const MMArgs a) {
             for (int w = 0; w < NW; ++w) s += gbuf[(size_t)w * nv + k];
             gv[k] = s * a.grad_scale;
         }
-        e = block_sum<NW>(ep, red());
+        e = block_sum<NW, double>(ep, red());
     };
 
     double e = 0.0;
@@ -118,7 +111,7 @@ __global__ void __launch_bounds__(NT) multimol_kernel(const MMArgs a) {
             const float *s_i = Sh + (size_t)sl * a.nv, *y_i = Yh + (size_t)sl * a.nv;
             double t = 0.0;
             for (int k = tid; k < n; k += NT) t += (double)s_i[k] * qv[k];
-            const double ai = (double)rho[sl] * block_sum<NW>(t, red());
+            const double ai = (double)rho[sl] * block_sum<NW, double>(t, red());
             if (tid == 0) alpha[i] = ai;
             const float af = (float)ai;
             for (int k = tid; k < n; k += NT) qv[k] -= af * y_i[k];
@@ -128,12 +121,12 @@ __global__ void __launch_bounds__(NT) multimol_kernel(const MMArgs a) {
         if (h > 0) {
             const int sl = (first + h - 1) % M;
             const float *s_l = Sh + (size_t)sl * a.nv, *y_l = Yh + (size_t)sl * a.nv;
-            double sy[2] = {0.0, 0.0}, z[1] = {0.0};
+            double sy[2] = {0.0, 0.0}, none[1];
             for (int k = tid; k < n; k += NT) {
                 sy[0] += (double)s_l[k] * y_l[k];
                 sy[1] += (double)y_l[k] * y_l[k];
             }
-            block_reduce<NW, 2, 1, double>(sy, z, red());
+            block_reduce<NW, 2, 0, double, double>(sy, none, red());
             gamma = sy[0] / (sy[1] + 1e-30);
         }
         const float gf = (float)gamma;
@@ -144,7 +137,7 @@ __global__ void __launch_bounds__(NT) multimol_kernel(const MMArgs a) {
             const float *s_i = Sh + (size_t)sl * a.nv, *y_i = Yh + (size_t)sl * a.nv;
             double t = 0.0;
             for (int k = tid; k < n; k += NT) t += (double)y_i[k] * qv[k];
-            const double beta = (double)rho[sl] * block_sum<NW>(t, red());
+            const double beta = (double)rho[sl] * block_sum<NW, double>(t, red());
             const float c = (float)(alpha[i] - beta);
             for (int k = tid; k < n; k += NT) qv[k] += s_i[k] * c;
             __syncthreads();
@@ -177,7 +170,7 @@ __global__ void __launch_bounds__(NT) multimol_kernel(const MMArgs a) {
             y_n[k] = y;
             t += (double)dv[k] * y;
         }
-        const double sy = block_sum<NW>(t, red());
+        const double sy = block_sum<NW, double>(t, red());
         if (tid == 0) rho[sl] = sy > kEpsCurv ? (float)(1.0 / (sy + 1e-30)) : 0.f;
         ++hcount;
         __threadfence_block();
@@ -196,7 +189,7 @@ __global__ void __launch_bounds__(NT) multimol_kernel(const MMArgs a) {
             const double v = sqrt(g0 * g0 + g1 * g1 + g2 * g2);
             mx[0] = v > mx[0] ? v : mx[0];
         }
-        block_reduce<NW, 1, 1, double>(z, mx, red());
+        block_reduce<NW, 1, 1, double, double>(z, mx, red());
         const bool improved = e < a.S.best_e[conf];
         if (improved)
             for (int k = tid; k < n; k += NT) BX[k] = xv[k];

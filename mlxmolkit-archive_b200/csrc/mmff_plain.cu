@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(NT) fused_sd_kernel(const Params P, float max_
     R alpha = grad_lr;
     A E = A(0), Eprev = A(1e30);
     for (int it = 0; it < P.max_iters; ++it) {
-        A e1[1] = {eval_terms<R, A, NW, true, true>(P, m, pos4, gbuf, ms, nv)}, z[1] = {A(0)};
+        A e1[1] = {eval_terms<R, A, NW, true, true>(P, m, pos4, gbuf, ms, nv)};
         __syncthreads();
         for (int k = tid; k < n; k += NT) {
             R s = R(0);
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(NT) fused_sd_kernel(const Params P, float max_
             for (int w = 0; w < NW; ++w) s += gbuf[(size_t)w * nv + k];
             g[k] = s;
         }
-        block_reduce<NW, 1, 1, A>(e1, z, red + rsel * NW * 8);
+        e1[0] = block_sum<NW, A>(e1[0], red + rsel * NW * 8);
         rsel ^= 1;
         E = (A)(float)e1[0];
         if (it > 0 && E > Eprev + A(1)) {
@@ -363,13 +363,13 @@ __global__ void __launch_bounds__(NT) fused_sd_kernel(const Params P, float max_
             continue;
         }
         if (it > 0) {
-            A s2[2] = {A(0), A(0)}, z2[1] = {A(0)};
+            A s2[2] = {A(0), A(0)}, none[1];
             for (int k = tid; k < n; k += NT) {
                 const R si = x[k] - pp[k], yi = g[k] - pg[k];
                 s2[0] += (A)(si * si);
                 s2[1] += (A)(si * yi);
             }
-            block_reduce<NW, 2, 1, A>(s2, z2, red + rsel * NW * 8);
+            block_reduce<NW, 2, 0, A, A>(s2, none, red + rsel * NW * 8);
             rsel ^= 1;
             if (s2[1] > A(1e-20)) alpha = fminf(fmaxf((float)(s2[0] / s2[1]), 1e-6f), 0.3f);
         }
