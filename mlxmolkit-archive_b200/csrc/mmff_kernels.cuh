@@ -794,6 +794,7 @@ struct Opt {
     uint32_t phase;    // parity of each of this warp's stages
     int *abort_flag;   // CTA-wide: a bounded wait gave up (shared memory)
     int ldh;           // row stride of H
+    bool ident;        // H is the identity and not written out (lean FP32 instances)
     bool use64;        // line-search energies in FP64 (escalated)
     int *cls;
     double *qa;
@@ -814,6 +815,7 @@ struct Opt {
         mbar = (uint64_t *)(sm + L.mbar);
         phase = 0;
         ldh = 0;
+        ident = false;
         xo = (R *)(sm + L.xo); dg = (R *)(sm + L.dg); hp = (R *)(sm + L.hp); hq = (R *)(sm + L.hq);
         pxi = (R *)(sm + L.pxi); pc = (R *)(sm + L.pc); pr = (R *)(sm + L.pr); gbuf = (R *)(sm + L.gbuf);
         cls = (int *)(sm + L.cls); qa = (double *)(sm + L.q); red = (A *)(sm + L.red);
@@ -923,6 +925,119 @@ struct Opt {
             while (!__all_sync(0xffffffffu, mbar_try_wait(&bw[st], (phase >> st) & 1u)) && ++spins < kDrainSpins) {
             }
             phase ^= 1u << st;
+        }
+    }
+
+    // Butterfly reduce-scatter of 8 per-lane partial sums (9 shuffles, each sum in the order of a
+    // full butterfly): lane l holds the warp-wide sum of value l >> 2.
+    static __device__ __forceinline__ float reduce8(const float (&v)[8]) {
+        const int lane = threadIdx.x & 31;
+        const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+        float w[4], x[2];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            w[k] = (b4 ? v[k + 4] : v[k]) + __shfl_xor_sync(0xffffffffu, b4 ? v[k] : v[k + 4], 16);
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            x[k] = (b3 ? w[k + 2] : w[k]) + __shfl_xor_sync(0xffffffffu, b3 ? w[k] : w[k + 2], 8);
+        float z = (b2 ? x[1] : x[0]) + __shfl_xor_sync(0xffffffffu, b2 ? x[0] : x[1], 4);
+        z += __shfl_xor_sync(0xffffffffu, z, 2);
+        return z + __shfl_xor_sync(0xffffffffu, z, 1);
+    }
+
+    // The pass while H is the identity (after the start or a restart): without a pending update the
+    // products are the vectors themselves; the first update makes the rows from the identity
+    // instead of reading them, so the identity is never written or read.  B200,
+    // 5000 conformers of 18-150 atoms x 5 iterations: 4.51 -> 3.83 ms, 12 % of which was writing the
+    // identity.
+    __device__ __forceinline__ void hpass_identity(bool pending) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        if (!pending) {
+            for (int k = threadIdx.x; k < n; k += NT) {
+                hp[k] = g[k] + R(0);   // -0 becomes the +0 of a sum
+                hq[k] = dg[k] + R(0);
+            }
+            return;
+        }
+        for (int i = warp; i < n; i += NW) {
+            float *row = (float *)mat + (size_t)i * ldh;
+            const float ri = pr[i], xi = pxi[i];
+            float ap = 0.0f, aq = 0.0f;
+            if constexpr (MSM) {
+                for (int j = lane; j < n; j += 32) {
+                    const float h = fmaf(xi, pc[j], fmaf(pxi[j], ri, i == j ? 1.0f : 0.0f));
+                    row[j] = h;
+                    ap = fmaf(h, g[j], ap);
+                    aq = fmaf(h, dg[j], aq);
+                }
+            } else {
+                const float4 *X4 = (const float4 *)pxi, *C4 = (const float4 *)pc;
+                const float4 *G4 = (const float4 *)g, *D4 = (const float4 *)dg;
+                for (int c = lane; 4 * c < ldh; c += 32) {
+                    const float4 px = X4[c], pv = C4[c], gg = G4[c], dd = D4[c];
+                    const int d = i - 4 * c;
+                    float4 h;
+                    h.x = fmaf(xi, pv.x, fmaf(px.x, ri, d == 0 ? 1.0f : 0.0f));
+                    h.y = fmaf(xi, pv.y, fmaf(px.y, ri, d == 1 ? 1.0f : 0.0f));
+                    h.z = fmaf(xi, pv.z, fmaf(px.z, ri, d == 2 ? 1.0f : 0.0f));
+                    h.w = fmaf(xi, pv.w, fmaf(px.w, ri, d == 3 ? 1.0f : 0.0f));
+                    reinterpret_cast<float4 *>(row)[c] = h;
+                    ap = fmaf(h.w, gg.w, fmaf(h.z, gg.z, fmaf(h.y, gg.y, fmaf(h.x, gg.x, ap))));
+                    aq = fmaf(h.w, dd.w, fmaf(h.z, dd.z, fmaf(h.y, dd.y, fmaf(h.x, dd.x, aq))));
+                }
+            }
+            ap = wsum(ap);
+            aq = wsum(aq);
+            if (lane == 0) { hp[i] = ap; hq[i] = aq; }
+        }
+        if (!MSM) fence_proxy_async_global();   // these stores before the next pass's TMA reads
+        ident = false;
+    }
+
+    // The pass of the lean FP32 instance with H in shared memory: four rows of a warp per step, so
+    // the update's and the products' vectors are read once for four rows, and the eight sums are
+    // reduced together.  25-48 atoms on B200: 38 % -> 29 % of an
+    // iteration, 14.2 -> 13.2 ms for 1207 conformers x 200 iterations.
+    __device__ __forceinline__ void hpass_rows4(bool pending) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        for (int i0 = warp; i0 < n; i0 += 4 * NW) {
+            float *row[4];
+            float r[4], x[4], v[8];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                // past the last row: the first of the group again, its results dropped
+                const int i = i0 + NW * u < n ? i0 + NW * u : i0;
+                row[u] = (float *)mat + (size_t)i * ldh;
+                r[u] = pending ? (float)pr[i] : 0.0f;
+                x[u] = pending ? (float)pxi[i] : 0.0f;
+                v[2 * u] = v[2 * u + 1] = 0.0f;
+            }
+            const int rows = (n - i0 + NW - 1) / NW;   // of this group and later ones
+            for (int j = lane; j < n; j += 32) {
+                const float gj = g[j], dj = dg[j];
+                float h[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) h[u] = row[u][j];
+                if (pending) {
+                    const float px = pxi[j], pv = pc[j];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        h[u] = fmaf(x[u], pv, fmaf(px, r[u], h[u]));
+                        if (u < rows) row[u][j] = h[u];
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    v[2 * u] = fmaf(h[u], gj, v[2 * u]);
+                    v[2 * u + 1] = fmaf(h[u], dj, v[2 * u + 1]);
+                }
+            }
+            const float sum = reduce8(v);
+            const int val = lane >> 2, u = val >> 1;
+            if ((lane & 3) == 0 && u < rows) {
+                if (val & 1) hq[i0 + NW * u] = sum;
+                else hp[i0 + NW * u] = sum;
+            }
         }
     }
 
@@ -1233,8 +1348,12 @@ struct Opt {
     }
 
     // inverse Hessian back to the identity (dense) / history cleared (L-BFGS)
+    // The lean FP32 instances note that H is the identity and write it with its first update.
+    static constexpr bool kLean = !LB && NC == 0 && sizeof(R) == 4;
     __device__ __forceinline__ void reset_matrix() {
-        if (!LB) {
+        if constexpr (kLean) {
+            ident = true;
+        } else if (!LB) {
             for (size_t e = threadIdx.x; e < (size_t)n * ldh; e += NT) {
                 const int i = (int)(e / ldh), j = (int)(e - (size_t)i * ldh);
                 mat[e] = i == j ? R(1) : R(0);
@@ -1427,8 +1546,11 @@ struct Opt {
                 }
                 if (!LB) {
                     __syncthreads();
-                    if constexpr (!MSM && NC == 0 && sizeof(R) == 4) hpass_stream_v4(pending);
-                    else if (MSM) hpass(pending);
+                    if constexpr (kLean) {
+                        if (ident) hpass_identity(pending);
+                        else if (MSM) hpass_rows4(pending);
+                        else hpass_stream_v4(pending);
+                    } else if (MSM) hpass(pending);
                     else hpass_stream(pending);
                     __syncthreads();
                     if (!MSM && *(volatile int *)abort_flag) { status = MMFFB_ST_TIMEOUT; break; }

@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(NT) fused_sd_kernel(const Params P, float max_
     using R = float;
     using A = double;
     const int conf = blockIdx.x, tid = threadIdx.x;
-    Layout L = make_layout(P.nmax, NW, 0, false, sizeof(R), sizeof(A), P.b.max_classes);
+    Layout L = make_layout(P.nmax, NW, 1, true, sizeof(R), sizeof(A), P.b.max_classes);
     R *pos4 = (R *)(smem + L.pos4), *x = (R *)(smem + L.x), *g = (R *)(smem + L.g);
     R *pp = (R *)(smem + L.xo), *pg = (R *)(smem + L.dg), *gbuf = (R *)(smem + L.gbuf);
     int *cls = (int *)(smem + L.cls);
@@ -468,7 +468,7 @@ int mmffb_fused_sd(const MMFFBatchDev *batch, const MMFFConfDev *confs, const MM
     P.pos = pos;
     P.energy = energy;
     constexpr int NT = 128;
-    Layout L = make_layout(P.nmax, NT / 32, 0, false, 4, 8, batch->max_classes);
+    Layout L = make_layout(P.nmax, NT / 32, 1, true, 4, 8, batch->max_classes);
     auto k = fused_sd_kernel<NT>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total);
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
