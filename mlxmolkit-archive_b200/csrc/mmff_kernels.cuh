@@ -260,6 +260,23 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 constexpr uint32_t kMaxWaitSpins = 1u << 22;   // bounded waits: give up, flag, never hang (default)
 constexpr uint32_t kDrainSpins = 1u << 22;     // bounded wait for copies still in flight after giving up
 
+// Two FP32 fused steps in one instruction (each lane of the pair rounds as fmaf does).
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
 template <class R> __device__ __forceinline__ R qprod(double a, double b);
 template <> __device__ __forceinline__ float qprod<float>(double a, double b) { return (float)(a * b); }
 // the term lists carry q_i*q_j rounded to float32 (mmff_params.py:305,318); every precision uses it
@@ -915,12 +932,12 @@ struct Opt {
         phase ^= 1u << st;
         return true;
     }
-    // After a wait gave up: bounded wait for this warp's copies of rows [from, to) still
-    // in flight -- the row whose wait gave up included -- so none lands in shared
+    // After a wait gave up: bounded wait for this warp's copies [from, to) still in flight
+    // -- the one whose wait gave up included -- so none lands in shared
     // memory after the CTA has moved on or exited.
-    __device__ __forceinline__ void drain(uint64_t *bw, int from, int to) {
+    __device__ __forceinline__ void drain(uint64_t *bw, int from, int to, int stages) {
         for (int t = from; t < to; ++t) {
-            const int st = t % kStages;
+            const int st = t % stages;
             uint32_t spins = 0;
             while (!__all_sync(0xffffffffu, mbar_try_wait(&bw[st], (phase >> st) & 1u)) && ++spins < kDrainSpins) {
             }
@@ -1123,7 +1140,7 @@ struct Opt {
         for (int t = 0; t < nrows; ++t) {
             const int st = t % kStages, i = warp + NW * t;
             if (!wait_stage(bw, st)) {
-                drain(bw, t, nrows < t + kStages ? nrows : t + kStages);
+                drain(bw, t, nrows < t + kStages ? nrows : t + kStages, kStages);
                 break;
             }
             const R *src = rw + (size_t)st * ldr;
@@ -1172,102 +1189,91 @@ struct Opt {
         fence_proxy_async_global();   // this pass's row stores before the next pass's TMA reads
     }
 
-    // The streamed pass of the register-lean FP32 instance: float4 columns (the
-    // rows of H and the vectors are padded to a multiple of 4 with zeros) and two
-    // rows per step, so each vector load from shared memory serves two rows and a
-    // warp keeps two row copies of its TMA ring in use at once.
+    // The streamed pass of the register-lean FP32 instance: float4 columns (the rows of H and the
+    // vectors are padded to a multiple of 4 with zeros) and two rows per step, so each vector load
+    // from shared memory serves two rows.  A warp's rows come in neighbouring pairs -- one copy, one
+    // wait and one ring stage for two rows -- and the update is two columns per instruction.  What
+    // bounds it is issue and the shared-memory loads, not the copies (more rows in flight, or plain
+    // 16-byte loads one pair ahead, measured no better; two pairs a stage 7 % slower at 49-100 atoms).
+    // B200, 200 iterations: 1209 conformers of 49-100 atoms 36.0 -> 31.0 ms, 1206 of 101-150 76.7 -> 67.0.
     __device__ __forceinline__ void hpass_stream_v4(bool pending) {
+        constexpr int kPairs = kStages / 2;    // row pairs in the ring
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        const int ldr = hld(3 * P.nmax);
-        float *rw = (float *)ring + (size_t)warp * kStages * ldr;
+        const int ldr = 2 * hld(3 * P.nmax);
+        float *rw = (float *)ring + (size_t)warp * kPairs * ldr;
         uint64_t *bw = mbar + warp * kStages;
-        const int nrows = warp < n ? (n - warp + NW - 1) / NW : 0;
+        const int all = (n + 1) >> 1, npairs = warp < all ? (all - warp + NW - 1) / NW : 0;
         const uint32_t bytes = (uint32_t)(ldh * sizeof(float));
         const int n4 = ldh >> 2;
-        const float4 *X4 = (const float4 *)pxi, *C4 = (const float4 *)pc;
+        const ulonglong2 *X4 = (const ulonglong2 *)pxi, *C4 = (const ulonglong2 *)pc;
         const float4 *G4 = (const float4 *)g, *D4 = (const float4 *)dg;
         float *H = (float *)mat;
-        if (lane == 0) {
-            for (int t = 0; t < nrows && t < kStages; ++t) {
-                mbar_expect_tx(&bw[t], bytes);
-                tma_load_row(rw + (size_t)t * ldr, H + (size_t)(warp + NW * t) * ldh, bytes, &bw[t]);
-            }
-        }
+        // copy of this warp's pair t into its stage (the last pair of an odd n is one row)
+        auto copy = [&](int t) {
+            const int st = t % kPairs, i = 2 * (warp + NW * t);
+            const uint32_t b = i + 1 < n ? 2 * bytes : bytes;
+            mbar_expect_tx(&bw[st], b);
+            tma_load_row(rw + (size_t)st * ldr, H + (size_t)i * ldh, b, &bw[st]);
+        };
+        if (lane == 0)
+            for (int t = 0; t < npairs && t < kPairs; ++t) copy(t);
         // groups of 4 row pairs: the 16 per-lane partial sums are reduced together
-        for (int t0 = 0; t0 < nrows; t0 += 8) {
+        for (int t0 = 0; t0 < npairs; t0 += 4) {
             float v[16];
 #pragma unroll
             for (int k = 0; k < 16; ++k) v[k] = 0.f;
             bool aborted = false;
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const int t = t0 + 2 * u;
-                if (t >= nrows) break;
-                const bool two = t + 1 < nrows;
-                const int s0 = t % kStages, s1 = (t + 1) % kStages;
-                const int issued = nrows < t + kStages ? nrows : t + kStages;
-                if (!wait_stage(bw, s0)) {
-                    drain(bw, t, issued);
+                const int t = t0 + u;
+                if (t >= npairs) break;
+                const int st = t % kPairs, i0 = 2 * (warp + NW * t);
+                const bool two = i0 + 1 < n;
+                if (!wait_stage(bw, st)) {
+                    drain(bw, t, npairs < t + kPairs ? npairs : t + kPairs, kPairs);
                     aborted = true;
                     break;
                 }
-                if (two && !wait_stage(bw, s1)) {
-                    drain(bw, t + 1, issued);
-                    aborted = true;
-                    break;
-                }
-                const int i0 = warp + NW * t, i1 = i0 + NW;
-                const float4 *A0 = (const float4 *)(rw + (size_t)s0 * ldr), *A1 = (const float4 *)(rw + (size_t)s1 * ldr);
-                float4 *W0 = (float4 *)(H + (size_t)i0 * ldh), *W1 = (float4 *)(H + (size_t)(two ? i1 : i0) * ldh);
+                const ulonglong2 *A0 = (const ulonglong2 *)(rw + (size_t)st * ldr);
+                const ulonglong2 *A1 = two ? A0 + n4 : A0;
+                ulonglong2 *W0 = (ulonglong2 *)(H + (size_t)i0 * ldh), *W1 = two ? W0 + n4 : W0;
                 const float r0 = pending ? (float)pr[i0] : 0.f, x0 = pending ? (float)pxi[i0] : 0.f;
-                const float r1 = (pending && two) ? (float)pr[i1] : 0.f, x1 = (pending && two) ? (float)pxi[i1] : 0.f;
+                const float r1 = (pending && two) ? (float)pr[i0 + 1] : 0.f;
+                const float x1 = (pending && two) ? (float)pxi[i0 + 1] : 0.f;
+                const uint64_t r00 = pack2(r0, r0), x00 = pack2(x0, x0), r11 = pack2(r1, r1), x11 = pack2(x1, x1);
                 float a0 = 0.f, q0 = 0.f, a1 = 0.f, q1 = 0.f;
                 for (int c = lane; c < n4; c += 32) {
-                    float4 h0 = A0[c];
-                    float4 h1 = two ? A1[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    ulonglong2 h0 = A0[c], h1 = A1[c];
                     if (pending) {
-                        const float4 px = X4[c], pv = C4[c];
-                        h0.x = fmaf(x0, pv.x, fmaf(px.x, r0, h0.x));
-                        h0.y = fmaf(x0, pv.y, fmaf(px.y, r0, h0.y));
-                        h0.z = fmaf(x0, pv.z, fmaf(px.z, r0, h0.z));
-                        h0.w = fmaf(x0, pv.w, fmaf(px.w, r0, h0.w));
+                        const ulonglong2 px = X4[c], pv = C4[c];
+                        h0.x = fma2(x00, pv.x, fma2(px.x, r00, h0.x));
+                        h0.y = fma2(x00, pv.y, fma2(px.y, r00, h0.y));
                         W0[c] = h0;
                         if (two) {
-                            h1.x = fmaf(x1, pv.x, fmaf(px.x, r1, h1.x));
-                            h1.y = fmaf(x1, pv.y, fmaf(px.y, r1, h1.y));
-                            h1.z = fmaf(x1, pv.z, fmaf(px.z, r1, h1.z));
-                            h1.w = fmaf(x1, pv.w, fmaf(px.w, r1, h1.w));
+                            h1.x = fma2(x11, pv.x, fma2(px.x, r11, h1.x));
+                            h1.y = fma2(x11, pv.y, fma2(px.y, r11, h1.y));
                             W1[c] = h1;
                         }
                     }
                     const float4 gg = G4[c], dd = D4[c];
-                    a0 = fmaf(h0.w, gg.w, fmaf(h0.z, gg.z, fmaf(h0.y, gg.y, fmaf(h0.x, gg.x, a0))));
-                    q0 = fmaf(h0.w, dd.w, fmaf(h0.z, dd.z, fmaf(h0.y, dd.y, fmaf(h0.x, dd.x, q0))));
-                    a1 = fmaf(h1.w, gg.w, fmaf(h1.z, gg.z, fmaf(h1.y, gg.y, fmaf(h1.x, gg.x, a1))));
-                    q1 = fmaf(h1.w, dd.w, fmaf(h1.z, dd.z, fmaf(h1.y, dd.y, fmaf(h1.x, dd.x, q1))));
+                    const float2 h0a = unpack2(h0.x), h0b = unpack2(h0.y), h1a = unpack2(h1.x), h1b = unpack2(h1.y);
+                    a0 = fmaf(h0b.y, gg.w, fmaf(h0b.x, gg.z, fmaf(h0a.y, gg.y, fmaf(h0a.x, gg.x, a0))));
+                    q0 = fmaf(h0b.y, dd.w, fmaf(h0b.x, dd.z, fmaf(h0a.y, dd.y, fmaf(h0a.x, dd.x, q0))));
+                    a1 = fmaf(h1b.y, gg.w, fmaf(h1b.x, gg.z, fmaf(h1a.y, gg.y, fmaf(h1a.x, gg.x, a1))));
+                    q1 = fmaf(h1b.y, dd.w, fmaf(h1b.x, dd.z, fmaf(h1a.y, dd.y, fmaf(h1a.x, dd.x, q1))));
                 }
                 v[4 * u] = a0; v[4 * u + 1] = q0; v[4 * u + 2] = a1; v[4 * u + 3] = q1;
-                __syncwarp();   // every lane's reads of both stages before they are refilled
-                if (lane == 0) {
+                __syncwarp();   // every lane's reads of the stage before it is refilled
+                if (lane == 0 && t + kPairs < npairs) {
                     fence_proxy_async_smem();
-                    if (t + kStages < nrows) {
-                        mbar_expect_tx(&bw[s0], bytes);
-                        tma_load_row(rw + (size_t)s0 * ldr, H + (size_t)(warp + NW * (t + kStages)) * ldh, bytes,
-                                     &bw[s0]);
-                    }
-                    if (t + 1 + kStages < nrows) {
-                        mbar_expect_tx(&bw[s1], bytes);
-                        tma_load_row(rw + (size_t)s1 * ldr, H + (size_t)(warp + NW * (t + 1 + kStages)) * ldh, bytes,
-                                     &bw[s1]);
-                    }
+                    copy(t + kPairs);
                 }
             }
             if (aborted) break;
             // lanes l and l^1 now hold the sum of value l >> 1: pair u = value / 4, then a0 q0 a1 q1
             const float sum = reduce16(v);
-            const int val = lane >> 1, tr = t0 + 2 * (val >> 2) + ((val >> 1) & 1);
-            if (!(lane & 1) && tr < nrows) {
-                const int i = warp + NW * tr;
+            const int val = lane >> 1, t = t0 + (val >> 2), i = 2 * (warp + NW * t) + ((val >> 1) & 1);
+            if (!(lane & 1) && t < npairs && i < n) {
                 if (val & 1) hq[i] = sum;
                 else hp[i] = sum;
             }
