@@ -618,14 +618,15 @@ __global__ void __launch_bounds__(NT) lbfgs_kernel(const __grid_constant__ Args 
                 ++hi;
                 if (hc < M) ++hc;
             }
-            // two-loop recursion (conformer_metal.py:518-545); rho is read after a reduction barrier
+            // two-loop recursion (conformer_metal.py:518-545)
             for (int i = tid; i < N; i += NT) Q[i] = G[i];
             for (int j = hc - 1; j >= 0; --j) {
                 int slot = (hi - 1 - (hc - 1 - j)) % M;
                 if (slot < 0) slot += M;
                 float t = 0.f;
                 for (int i = tid; i < N; i += NT) t += dot4(S[(size_t)slot * NA + i], Q[i]);
-                const float aj = rho[slot] * bsum<NT>(t, rb());
+                t = bsum<NT>(t, rb());        // its barrier publishes the newest rho
+                const float aj = __fmul_rn(rho[slot], t);
                 alph[j] = aj;
                 for (int i = tid; i < N; i += NT) Q[i] = axpy(-aj, Y[(size_t)slot * NA + i], Q[i]);
             }
@@ -647,7 +648,8 @@ __global__ void __launch_bounds__(NT) lbfgs_kernel(const __grid_constant__ Args 
                 if (slot < 0) slot += M;
                 float t = 0.f;
                 for (int i = tid; i < N; i += NT) t += dot4(Y[(size_t)slot * NA + i], Q[i]);
-                const float beta = rho[slot] * bsum<NT>(t, rb());
+                t = bsum<NT>(t, rb());
+                const float beta = __fmul_rn(rho[slot], t);
                 for (int i = tid; i < N; i += NT) Q[i] = axpy(alph[j] - beta, S[(size_t)slot * NA + i], Q[i]);
             }
             for (int i = tid; i < N; i += NT) D[i] = scale4(-1.0f, Q[i]);
