@@ -58,21 +58,35 @@ def _torch():
     return torch
 
 
+def _upload(arrays, device):
+    """Device tensors of ``arrays``: one buffer and one copy, complete on return (any stream may use
+    them), each array on a 512-byte boundary (the bonded records' alignment)."""
+    torch = _torch()
+    arrays = [np.ascontiguousarray(a).reshape(-1) for a in arrays]
+    starts = [0]
+    for a in arrays:
+        starts.append((starts[-1] + a.nbytes + 511) & ~511)
+    host = np.empty(max(starts[-1], 1), dtype=np.uint8)
+    for a, o in zip(arrays, starts):
+        host[o:o + a.nbytes] = a.view(np.uint8)
+    dev = torch.from_numpy(host).to(device, non_blocking=False)
+    return [dev[o:o + a.nbytes].view(getattr(torch, a.dtype.name)) for a, o in zip(arrays, starts)]
+
+
 class DeviceBatch:
     """Packed molecule tables resident in device memory (one upload, many launches)."""
 
-    def __init__(self, packed: PackedBatch, device=None):
+    def __init__(self, packed: PackedBatch, device=None, also=()):
+        """``also``: further arrays for the same upload (their tensors: ``self.also``)."""
         torch = _torch()
         self.packed = packed
         dev = device or torch.device("cuda", torch.cuda.current_device())
         self.device = dev
-        t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(dev, non_blocking=False)
-        self.mol_desc = t(packed.mol_desc.reshape(-1))
-        self.bonded = t(packed.bonded.view(np.int32).reshape(-1))
-        self.atom_cls = t(packed.atom_cls if len(packed.atom_cls) else np.zeros(1, np.int32))
-        self.atom_q = t(packed.atom_q if len(packed.atom_q) else np.zeros(1, np.float64))
-        self.cls_tab = t(packed.cls_tab.reshape(-1))
-        self.pair_mask = t(packed.pair_mask.view(np.int32))
+        (self.mol_desc, self.bonded, self.atom_cls, self.atom_q, self.cls_tab, self.pair_mask, *self.also) = _upload(
+            [packed.mol_desc, packed.bonded.view(np.int32),
+             packed.atom_cls if len(packed.atom_cls) else np.zeros(1, np.int32),
+             packed.atom_q if len(packed.atom_q) else np.zeros(1, np.float64),
+             packed.cls_tab, packed.pair_mask.view(np.int32), *also], dev)
         self.n_atoms = packed.n_atoms
         self.nbytes = sum(x.numel() * x.element_size() for x in (self.mol_desc, self.bonded, self.atom_cls,
                                                                   self.atom_q, self.cls_tab, self.pair_mask))
@@ -92,16 +106,21 @@ class DeviceConformers:
     """Conformer -> molecule map, coordinate offsets and processing order on the device."""
 
     def __init__(self, batch: DeviceBatch, conf_mol: np.ndarray, conf_coord: np.ndarray,
-                 order: Optional[np.ndarray] = None):
-        torch = _torch()
-        dev = batch.device
+                 order: Optional[np.ndarray] = None, on_dev=None):
+        """``on_dev``: the arrays' device tensors, when already uploaded (``arrays``)."""
         self.n_conf = int(len(conf_mol))
         self.conf_mol_np = np.asarray(conf_mol, dtype=np.int32)
         self.max_atoms = int(batch.n_atoms[self.conf_mol_np].max()) if self.n_conf else 1
-        self.conf_mol = torch.from_numpy(self.conf_mol_np.copy()).to(dev)
-        self.conf_coord = torch.from_numpy(np.asarray(conf_coord, dtype=np.int64).copy()).to(dev)
-        self.order = None if order is None else torch.from_numpy(np.asarray(order, np.int32).copy()).to(dev)
+        if on_dev is None:
+            on_dev = _upload(self.arrays(conf_mol, conf_coord, order), batch.device)
+        self.conf_mol, self.conf_coord = on_dev[:2]
+        self.order = None if order is None else on_dev[2]
         self.nbytes = 12 * self.n_conf + (0 if order is None else 4 * len(order))
+
+    @staticmethod
+    def arrays(conf_mol, conf_coord, order=None):
+        a = [np.asarray(conf_mol, dtype=np.int32), np.asarray(conf_coord, dtype=np.int64)]
+        return a if order is None else a + [np.asarray(order, np.int32)]
 
     def desc(self) -> _lib.MMFFConfDev:
         return _lib.MMFFConfDev(self.n_conf, self.max_atoms, self.conf_mol.data_ptr(),
@@ -186,11 +205,12 @@ class Minimizer:
             self.pack_s = time.perf_counter() - t
         else:
             self.pack_s = 0.0
-        self.batch = DeviceBatch(packed, device)
         n_atoms = [int(v) for v in packed.n_atoms]
         self.conf_mol, self.conf_coord, self.total = conformer_index(n_atoms, self.conf_counts)
         self.order = lpt_order(n_atoms, self.conf_mol)
-        self.confs = DeviceConformers(self.batch, self.conf_mol, self.conf_coord, self.order)
+        index = DeviceConformers.arrays(self.conf_mol, self.conf_coord, self.order)
+        self.batch = DeviceBatch(packed, device, also=index)
+        self.confs = DeviceConformers(self.batch, self.conf_mol, self.conf_coord, self.order, self.batch.also)
         self._scratch = None
         # host -> device bytes of the set-up (tables and conformer index arrays)
         self.upload_bytes = self.batch.nbytes + self.confs.nbytes
@@ -256,15 +276,15 @@ class Minimizer:
         return MinimizeResult(pos_dev.cpu().numpy(), e.cpu().numpy(), st.cpu().numpy(), it.cpu().numpy(),
                               e64.cpu().numpy(), de.cpu().numpy(), gr.cpu().numpy())
 
-    def fp64_check_device(self, pos_dev, energy_dev, mode=MODE_TG, stream=None):
+    def fp64_check_device(self, pos_dev, energy_dev, mode=MODE_TG, stream=None, out=None):
         """FP64 energy, error of ``energy_dev`` against it, and FP64 RMS gradient of every
-        conformer at ``pos_dev`` (device tensors, stream-ordered)."""
+        conformer at ``pos_dev`` (device tensors, stream-ordered; ``out``: the three to fill)."""
         torch = _torch()
         L = _lib.load()
         C = self.confs.n_conf
-        e64 = torch.empty(C, dtype=torch.float64, device=self.batch.device)
-        de = torch.empty(C, dtype=torch.float64, device=self.batch.device)
-        gr = torch.empty(C, dtype=torch.float64, device=self.batch.device)
+        if out is None:
+            out = tuple(torch.empty(C, dtype=torch.float64, device=self.batch.device) for _ in range(3))
+        e64, de, gr = out
         md = (ctypes.c_double * 4)(*[float(v) for v in mode])
         bd, cd = self.batch.desc(), self.confs.desc()
         rc = L.mmffb_fp64_check(ctypes.byref(bd), ctypes.byref(cd), md, pos_dev.data_ptr(), energy_dev.data_ptr(),
@@ -536,6 +556,15 @@ def launch_chunks(n_atoms, conf_counts, bins=DEFAULT_BINS, head_frac: float = 0.
     return chunks
 
 
+def _result_views(buf, c: int):
+    """The parts of a chunk's result buffer of c conformers: energies, FP64 energies, energy errors
+    and RMS gradients (float64), statuses and iterations (int32), the error word (one int32)."""
+    torch = _torch()
+    f = buf[:32 * c].view(torch.float64)
+    i = buf[32 * c:40 * c + 4].view(torch.int32)
+    return f[:c], f[c:2 * c], f[2 * c:3 * c], f[3 * c:], i[:c], i[c:2 * c], i[2 * c:]
+
+
 def minimize_pipelined(params_list, conf_counts, positions, *, max_iters: int, grad_tol: float = 1e-4,
                        history_m: int = 0, device=None) -> MinimizeResult:
     """The drop-in call's body: pack, upload and launch chunk by chunk (``launch_chunks``).
@@ -587,27 +616,31 @@ def minimize_pipelined(params_list, conf_counts, positions, *, max_iters: int, g
             xh = torch.from_numpy(np.concatenate([pos[coord0[i]:coord0[i + 1]] for i in idx])).pin_memory()
             x = torch.empty(xh.numel(), dtype=torch.float32, device=dev)
             x.copy_(xh, non_blocking=True)
-            err = torch.zeros(1, dtype=torch.int32, device=dev)
-            e, st, it = m.minimize_device(x, max_iters=max_iters, grad_tol=grad_tol, history_m=history_m,
-                                          err=err, stream=s)
+            # energies, FP64 checks, statuses, iterations and the launch's error word (which its
+            # start zeroes): one device buffer, read back by one copy
+            c_r = m.confs.n_conf
+            res = torch.empty(40 * c_r + 4, dtype=torch.uint8, device=dev)
+            e, e64, de, gr, st, it, err = _result_views(res, c_r)
+            m.minimize_device(x, max_iters=max_iters, grad_tol=grad_tol, history_m=history_m, out=(e, st, it),
+                              err=err, stream=s)
             if t_first is None:
                 t_first = time.perf_counter()
-            e64, de, gr = m.fp64_check_device(x, e, stream=s)
-            host = [torch.empty(t.shape, dtype=t.dtype, pin_memory=True) for t in (x, e, st, it, e64, de, gr, err)]
-            for h, t in zip(host, (x, e, st, it, e64, de, gr, err)):
+            m.fp64_check_device(x, e, stream=s, out=(e64, de, gr))
+            host = [torch.empty(t.shape, dtype=t.dtype, pin_memory=True) for t in (x, res)]
+            for h, t in zip(host, (x, res)):
                 h.copy_(t, non_blocking=True)
             done = torch.cuda.Event()
             done.record(s)
         upload += m.upload_bytes          # tables and conformer index arrays (coordinates apart)
-        live.append((idx, m, done, host, (x, e, st, it, e64, de, gr, err)))
+        live.append((idx, m, done, host, (x, res)))
     out_pos = np.empty(pos.size, dtype=np.float32)
     outs = [np.empty(C, dtype=np.float64), np.empty(C, dtype=np.int32), np.empty(C, dtype=np.int32),
             np.empty(C, dtype=np.float64), np.empty(C, dtype=np.float64), np.empty(C, dtype=np.float64)]
     gave_up, bad = False, 0
     for idx, m, done, host, _ in live:
         done.synchronize()
-        hx, he, hst, hit, he64, hde, hgr, herr = (h.numpy() for h in host)
-        out_pos[_ranges(coord0[idx], sizes[idx])] = hx
+        he, he64, hde, hgr, hst, hit, herr = (h.numpy() for h in _result_views(host[1], m.confs.n_conf))
+        out_pos[_ranges(coord0[idx], sizes[idx])] = host[0].numpy()
         cidx = _ranges(conf0[idx], k[idx])
         for o, h in zip(outs, (he, hst, hit, he64, hde, hgr)):
             o[cidx] = h

@@ -306,11 +306,13 @@ def pack_molecules(params_list, n_threads: int = 0) -> PackedBatch:
     keep = []
 
     def arr(xs, dt):
-        a = np.ascontiguousarray(np.concatenate(xs) if xs else np.zeros(1), dtype=dt)
+        # one molecule's arrays are read where they are
+        joined = xs[0] if len(xs) == 1 else np.concatenate(xs) if xs else np.zeros(1)
+        a = np.ascontiguousarray(joined, dtype=dt)
         if a.size == 0:
             a = np.zeros(1, dtype=dt)
         keep.append(a)
-        return a.ctypes.data
+        return a.__array_interface__["data"][0]
 
     counts = np.array([[len(getattr(p, f)) for f in _TERM_COUNT_FIELDS] for p in params_list],
                       dtype=np.int64).reshape(M, 7)
