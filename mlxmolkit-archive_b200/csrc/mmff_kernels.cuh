@@ -365,9 +365,9 @@ __device__ __forceinline__ float u2f(uint32_t u) { return __uint_as_float(u); }
 
 // Per-conformer molecule data staged in shared memory.
 struct MolSmem {
-    const int *cls;        // non-bonded class per atom
+    const int *cls;        // non-bonded class per atom, times 8 (a byte offset into a table row)
     const double *qa;      // partial charge per atom (FP64; FP32 evaluations take it from pos4)
-    const uint32_t *mask;  // N x W non-bonded-pair bit rows, then N x W 1-4 bit rows
+    const uint2 *mask;     // N x W words of the non-bonded-pair bit rows (x) and the 1-4 rows (y)
     const float2 *tab;     // ncls x ncls (R*, eps)
 };
 
@@ -379,21 +379,29 @@ template <> __device__ __forceinline__ void ld3<float>(const float *p4, int a, f
     x = v.x; y = v.y; z = v.z;
 }
 
+// The class table's row of the class at offset cls8, and the row's entry of another.
+__device__ __forceinline__ const char *table_row(const float2 *tab, int cls8, int ncls) {
+    return reinterpret_cast<const char *>(tab) + cls8 * ncls;
+}
+__device__ __forceinline__ float2 table_at(const char *row, int cls8) {
+    return *reinterpret_cast<const float2 *>(row + cls8);
+}
+
 // Copy a molecule's bit rows, class table, classes and charges into shared memory.
 // IR (the FP32 instances): stage 1/R* in place of R*, the pair term's only use of R*.
 // pos4 (FP32 instances): its fourth component takes the atom's charge, read with the position.
 template <int NT, bool IR = false>
 __device__ __forceinline__ void stage_molecule(const Params &P, const MolV &m, int *cls, double *qa, float *pos4,
-                                               uint32_t *mask, float2 *tab) {
+                                               uint2 *mask, float2 *tab) {
     const int N = m.n, W = (N + 31) >> 5;
     for (int a = threadIdx.x; a < N; a += NT) {
-        cls[a] = __ldcg(P.b.atom_cls + m.atom_off + a);
+        cls[a] = 8 * __ldcg(P.b.atom_cls + m.atom_off + a);
         const double q = __ldcg(P.b.atom_q + m.atom_off + a);
         qa[a] = q;
         if (IR) pos4[4 * a + 3] = (float)q;
     }
     const uint32_t *gm = P.b.pair_mask + m.mask_off;
-    for (int k = threadIdx.x; k < 2 * N * W; k += NT) mask[k] = __ldcg(gm + k);
+    for (int k = threadIdx.x; k < N * W; k += NT) mask[k] = make_uint2(__ldcg(gm + k), __ldcg(gm + N * W + k));
     const float2 *gt = reinterpret_cast<const float2 *>(P.b.cls_tab) + m.cls_off;
     for (int k = threadIdx.x; k < m.ncls * m.ncls; k += NT) {
         float2 v = __ldcg(gt + k);
@@ -427,7 +435,9 @@ __device__ __forceinline__ void scatter_rows(const float (&f)[3], const float (&
 // G, their forces to the warp's buffer gw.  Bound by instruction issue at 16 warps an SM: the
 // hardware reciprocals without denormal steps, charges read with the positions, the dielectric
 // chosen outside the loop and 8 instead of 30 shuffles for two rows' sums took 672 conformers of
-// 131-369 atoms x 8 L-BFGS iterations from 2.39 to 2.15 ms, 5000 drug-like x 5 from 4.83 to 4.70.
+// 131-369 atoms x 8 L-BFGS iterations from 2.39 to 2.15 ms, 5000 drug-like x 5 from 4.83 to 4.70;
+// pair and 1-4 bits in one word pair, class offsets in bytes and running pointers (71.5 -> 68.3 M
+// warp instructions for 444 evaluations of 280 atoms) from 1.96 to 1.79 and 3.59 to 3.48.
 template <class A, int NW, bool G, bool DD>
 __device__ __forceinline__ A pair_rows(const MolV &m, const float *pos4, float *gw, const MolSmem &ms, A acc) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -436,28 +446,29 @@ __device__ __forceinline__ A pair_rows(const MolV &m, const float *pos4, float *
     // Non-bonded pairs, implicit from the staged bit rows and class table: rows i and i + NW per
     // step, lanes over the columns, so two independent pair chains per lane and one scatter per
     // column (a pair absent from the bit rows contributes nothing).
+    // (A row's words below its first column are zero, and row N - 1 is all zero: it stands in where
+    // there is no second row.)
     const int W = (N + 31) >> 5;
-    const uint32_t *pm = ms.mask, *p14 = ms.mask + (size_t)N * W;
     const float4 *X = reinterpret_cast<const float4 *>(pos4);
     for (int i = warp; i < N - 1; i += 2 * NW) {
         const int i2 = i + NW;
         const bool has2 = i2 < N - 1;
-        const int ik = has2 ? i2 : i;
+        const int ik = has2 ? i2 : N - 1;
         const float4 a = X[i], b = X[ik];
-        const float2 *ti = ms.tab + ms.cls[i] * m.ncls, *tk = ms.tab + ms.cls[ik] * m.ncls;
-        const uint32_t *mi = pm + i * W, *mk = pm + ik * W, *ni = p14 + i * W, *nk = p14 + ik * W;
+        const char *ti = table_row(ms.tab, ms.cls[i], m.ncls), *tk = table_row(ms.tab, ms.cls[ik], m.ncls);
         float f[3] = {0.0f, 0.0f, 0.0f}, k[3] = {0.0f, 0.0f, 0.0f};
-        const int w2 = has2 ? (i2 + 1) >> 5 : W;   // the second row's first word
-        for (int wb = (i + 1) >> 5; wb < W; ++wb) {
-            const uint32_t wd = mi[wb], wd2 = wb >= w2 ? mk[wb] : 0u;
-            const bool b1 = (wd & bit) != 0u, b2 = (wd2 & bit) != 0u;
+        const int wb0 = (i + 1) >> 5;
+        const uint2 *mi = ms.mask + i * W + wb0, *mk = ms.mask + ik * W + wb0, *end = ms.mask + (i + 1) * W;
+        for (int j = 32 * wb0 + lane; mi < end; ++mi, ++mk, j += 32) {
+            const uint2 wi = *mi, wk = *mk;
+            const bool b1 = (wi.x & bit) != 0u, b2 = (wk.x & bit) != 0u;
             if (b1 || b2) {
-                const int j = 32 * wb + lane, cj = ms.cls[j];
-                const float2 t1 = ti[cj], t2 = tk[cj];
+                const int cj = ms.cls[j];
+                const float2 t1 = table_at(ti, cj), t2 = table_at(tk, cj);
                 const float4 x = X[j];
                 float q1 = __fmul_rn(a.w, x.w), q2 = __fmul_rn(b.w, x.w);
-                if (ni[wb] & bit) q1 = __fmul_rn(q1, 0.75f);
-                if (nk[wb] & bit) q2 = __fmul_rn(q2, 0.75f);
+                if (wi.y & bit) q1 = __fmul_rn(q1, 0.75f);
+                if (wk.y & bit) q2 = __fmul_rn(q2, 0.75f);
                 const float dx1 = a.x - x.x, dy1 = a.y - x.y, dz1 = a.z - x.z;
                 const float dx2 = b.x - x.x, dy2 = b.y - x.y, dz2 = b.z - x.z;
                 float ev1, ee1, s1, ev2, ee2, s2;
@@ -725,7 +736,6 @@ __device__ __forceinline__ A eval_terms(const Params &P, const MolV &m, const R 
 
     // non-bonded pairs, implicit from the staged bit rows and class table
     const int W = (N + 31) >> 5;
-    const uint32_t *pm = ms.mask, *p14 = ms.mask + (size_t)N * W;
     const bool dd = m.diel == 2;
     // Rows i and i + NW per step: two independent pair chains per lane (both are
     // evaluated; a pair absent from the bit rows contributes nothing) and one
@@ -736,21 +746,21 @@ __device__ __forceinline__ A eval_terms(const Params &P, const MolV &m, const R 
         R xi, yi, zi, xk = R(0), yk = R(0), zk = R(0);
         ld3(pos4, i, xi, yi, zi);
         if (has2) ld3(pos4, i2, xk, yk, zk);
-        const int ci = ms.cls[i] * m.ncls, ck = has2 ? ms.cls[i2] * m.ncls : 0;
+        const char *ti = table_row(ms.tab, ms.cls[i], m.ncls), *tk = table_row(ms.tab, has2 ? ms.cls[i2] : 0, m.ncls);
         const int ik = has2 ? i2 : i;
         R fx = R(0), fy = R(0), fz = R(0), kx = R(0), ky = R(0), kz = R(0);
         const int jb2 = has2 ? ((i2 + 1) & ~31) : N;
         for (int jb = (i + 1) & ~31; jb < N; jb += 32) {
             const int wb = jb >> 5;
-            const uint32_t wd = pm[i * W + wb];
-            const uint32_t wd2 = jb >= jb2 ? pm[i2 * W + wb] : 0u;
+            const uint2 wi = ms.mask[i * W + wb], wk = jb >= jb2 ? ms.mask[i2 * W + wb] : make_uint2(0u, 0u);
+            const uint32_t wd = wi.x, wd2 = wk.x;
             if ((wd | wd2) == 0u) continue;
             const bool b1 = (wd >> lane) & 1u, b2 = (wd2 >> lane) & 1u;
             if (b1 || b2) {
                 const int j = jb + lane;
                 const int cj = ms.cls[j];
-                const float2 t1 = ms.tab[ci + cj], t2 = ms.tab[ck + cj];
-                const uint32_t w14 = p14[i * W + wb], w14b = jb >= jb2 ? p14[i2 * W + wb] : 0u;
+                const float2 t1 = table_at(ti, cj), t2 = table_at(tk, cj);
+                const uint32_t w14 = wi.y, w14b = wk.y;
                 R q1 = qprod<R>(ms.qa[i], ms.qa[j]), q2 = qprod<R>(ms.qa[ik], ms.qa[j]);
                 if ((w14 >> lane) & 1u) q1 *= R(0.75);
                 if ((w14b >> lane) & 1u) q2 *= R(0.75);
@@ -815,7 +825,7 @@ struct Opt {
     bool use64;        // line-search energies in FP64 (escalated)
     int *cls;
     double *qa;
-    uint32_t *mask;
+    uint2 *mask;
     float2 *tab;
     MolSmem ms;
     A *red, *rho_s, *alpha_s;
@@ -836,7 +846,7 @@ struct Opt {
         xo = (R *)(sm + L.xo); dg = (R *)(sm + L.dg); hp = (R *)(sm + L.hp); hq = (R *)(sm + L.hq);
         pxi = (R *)(sm + L.pxi); pc = (R *)(sm + L.pc); pr = (R *)(sm + L.pr); gbuf = (R *)(sm + L.gbuf);
         cls = (int *)(sm + L.cls); qa = (double *)(sm + L.q); red = (A *)(sm + L.red);
-        mask = (uint32_t *)(sm + L.mask); tab = (float2 *)(sm + L.tab);
+        mask = (uint2 *)(sm + L.mask); tab = (float2 *)(sm + L.tab);
         ms.cls = cls; ms.qa = qa; ms.mask = mask; ms.tab = tab;
         rho_s = (A *)(sm + L.rho); alpha_s = (A *)(sm + L.alpha);
         if (MSM) mat = (R *)(sm + L.mat);
@@ -1771,7 +1781,7 @@ __global__ void __launch_bounds__(NT) energy_grad_kernel(const Params P, float *
     R *pos4 = (R *)(smem + L.pos4), *gbuf = (R *)(smem + L.gbuf);
     int *cls = (int *)(smem + L.cls);
     double *qa = (double *)(smem + L.q);
-    uint32_t *mask = (uint32_t *)(smem + L.mask);
+    uint2 *mask = (uint2 *)(smem + L.mask);
     float2 *tab = (float2 *)(smem + L.tab);
     A *red = (A *)(smem + L.red);
     const MolV m = load_mol(P.b.mol_desc, P.c.conf_mol[conf]);
@@ -1812,7 +1822,7 @@ __global__ void __launch_bounds__(NT) check64_kernel(const Params P, const doubl
     double *pos4 = (double *)(smem + L.pos4), *gbuf = (double *)(smem + L.gbuf);
     int *cls = (int *)(smem + L.cls);
     double *qa = (double *)(smem + L.q);
-    uint32_t *mask = (uint32_t *)(smem + L.mask);
+    uint2 *mask = (uint2 *)(smem + L.mask);
     float2 *tab = (float2 *)(smem + L.tab);
     double *red = (double *)(smem + L.red);
     const MolV m = load_mol(P.b.mol_desc, P.c.conf_mol[conf]);

@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(NT) multimol_kernel(const MMArgs a) {
     float *qv = (float *)(smem + L.hq);
     int *cls = (int *)(smem + L.cls);
     double *qa = (double *)(smem + L.q);
-    uint32_t *mask = (uint32_t *)(smem + L.mask);
+    uint2 *mask = (uint2 *)(smem + L.mask);
     float2 *tab = (float2 *)(smem + L.tab);
     double *red0 = (double *)(smem + L.red), *red1 = red0 + NW * 8;
     double *alpha = (double *)(smem + L.alpha);

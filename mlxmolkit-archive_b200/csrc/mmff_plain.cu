@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(NT) fused_sd_kernel(const Params P, float max_
     R *pp = (R *)(smem + L.xo), *pg = (R *)(smem + L.dg), *gbuf = (R *)(smem + L.gbuf);
     int *cls = (int *)(smem + L.cls);
     double *qa = (double *)(smem + L.q);
-    uint32_t *mask = (uint32_t *)(smem + L.mask);
+    uint2 *mask = (uint2 *)(smem + L.mask);
     float2 *tab = (float2 *)(smem + L.tab);
     A *red = (A *)(smem + L.red);
     int rsel = 0;
