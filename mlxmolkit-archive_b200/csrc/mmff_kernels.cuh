@@ -523,8 +523,14 @@ __device__ __forceinline__ A eval_terms32(const Params &P, const MolV &m, const 
     }
     const uint4 *BR = reinterpret_cast<const uint4 *>(P.b.bonded);
     const t32::Mode md(P.md);
+    // The warp's first chunk of a term type.  With gradients chunk c is warp c mod NW's, whose buffer
+    // sums a fixed sequence; an energy alone deals the chunks of all types in one round, so that a
+    // small molecule's few chunks do not all fall to the first warps (2500 conformers of 23-72 atoms x 5
+    // iterations: 1.28 -> 1.25 ms on B200).
+    const auto first = [&](int before) { return G ? warp : (warp + NW - before % NW) % NW; };
+    const int anch0 = m.bnch, snch0 = anch0 + m.anch, onch0 = snch0 + m.snch, tnch0 = onch0 + m.onch;
 
-    for (int c = warp; c < m.bnch; c += NW) {
+    for (int c = first(0); c < m.bnch; c += NW) {
         const uint4 r = __ldg(BR + m.boff + (size_t)c * 32 + lane);
         const bool v = r.x != 0xffffffffu;
         const int i = r.x & 0xffff, j = r.x >> 16;
@@ -540,7 +546,7 @@ __device__ __forceinline__ A eval_terms32(const Params &P, const MolV &m, const 
             __syncwarp();
         }
     }
-    for (int c = warp; c < m.anch; c += NW) {
+    for (int c = first(anch0); c < m.anch; c += NW) {
         const uint4 r = __ldg(BR + m.aoff + (size_t)c * 32 + lane);
         const bool v = r.x != 0xffffffffu;
         const int i = r.x & 0xffff, j = r.x >> 16, k = r.y & 0xffff;
@@ -560,7 +566,7 @@ __device__ __forceinline__ A eval_terms32(const Params &P, const MolV &m, const 
             __syncwarp();
         }
     }
-    for (int c = warp; c < m.snch; c += NW) {
+    for (int c = first(snch0); c < m.snch; c += NW) {
         const uint4 r0 = __ldg(BR + m.soff + (size_t)c * 64 + lane);
         const uint4 r1 = __ldg(BR + m.soff + (size_t)c * 64 + 32 + lane);
         const bool v = r0.x != 0xffffffffu;
@@ -579,7 +585,7 @@ __device__ __forceinline__ A eval_terms32(const Params &P, const MolV &m, const 
             __syncwarp();
         }
     }
-    for (int c = warp; c < m.onch; c += NW) {
+    for (int c = first(onch0); c < m.onch; c += NW) {
         const uint4 r = __ldg(BR + m.ooff + (size_t)c * 32 + lane);
         const bool v = r.x != 0xffffffffu;
         const int i = r.x & 0xffff, j = r.x >> 16, k = r.y & 0xffff, l = r.y >> 16;
@@ -600,7 +606,7 @@ __device__ __forceinline__ A eval_terms32(const Params &P, const MolV &m, const 
             __syncwarp();
         }
     }
-    for (int c = warp; c < m.tnch; c += NW) {
+    for (int c = first(tnch0); c < m.tnch; c += NW) {
         const uint4 r0 = __ldg(BR + m.toff + (size_t)c * 64 + lane);
         const uint4 r1 = __ldg(BR + m.toff + (size_t)c * 64 + 32 + lane);
         const bool v = r0.x != 0xffffffffu;
