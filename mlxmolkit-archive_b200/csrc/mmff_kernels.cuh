@@ -827,7 +827,7 @@ struct Opt {
     uint32_t phase;    // parity of each of this warp's stages
     int *abort_flag;   // CTA-wide: a bounded wait gave up (shared memory)
     int ldh;           // row stride of H
-    bool ident;        // H is the identity and not written out (lean FP32 instances)
+    bool ident;        // H is the identity and not written out
     bool use64;        // line-search energies in FP64 (escalated)
     int *cls;
     double *qa;
@@ -982,7 +982,7 @@ struct Opt {
     // products are the vectors themselves; the first update makes the rows from the identity
     // instead of reading them, so the identity is never written or read.  B200,
     // 5000 conformers of 18-150 atoms x 5 iterations: 4.51 -> 3.83 ms, 12 % of which was writing the
-    // identity.
+    // identity; 504 FP64 conformers of 18-110 atoms x 15: 3.12 -> 2.75 ms.
     __device__ __forceinline__ void hpass_identity(bool pending) {
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         if (!pending) {
@@ -993,15 +993,15 @@ struct Opt {
             return;
         }
         for (int i = warp; i < n; i += NW) {
-            float *row = (float *)mat + (size_t)i * ldh;
-            const float ri = pr[i], xi = pxi[i];
-            float ap = 0.0f, aq = 0.0f;
-            if constexpr (MSM) {
+            R *row = mat + (size_t)i * ldh;
+            const R ri = pr[i], xi = pxi[i];
+            R ap = R(0), aq = R(0);
+            if constexpr (MSM || !kLean) {
                 for (int j = lane; j < n; j += 32) {
-                    const float h = fmaf(xi, pc[j], fmaf(pxi[j], ri, i == j ? 1.0f : 0.0f));
+                    const R h = fma(xi, pc[j], fma(pxi[j], ri, i == j ? R(1) : R(0)));
                     row[j] = h;
-                    ap = fmaf(h, g[j], ap);
-                    aq = fmaf(h, dg[j], aq);
+                    ap = fma(h, g[j], ap);
+                    aq = fma(h, dg[j], aq);
                 }
             } else {
                 const float4 *X4 = (const float4 *)pxi, *C4 = (const float4 *)pc;
@@ -1369,19 +1369,11 @@ struct Opt {
         }
     }
 
-    // inverse Hessian back to the identity (dense) / history cleared (L-BFGS)
-    // The lean FP32 instances note that H is the identity and write it with its first update.
+    // Inverse Hessian back to the identity: noted, and written with its first update (L-BFGS: the
+    // caller's empty history is all there is to it).
     static constexpr bool kLean = !LB && NC == 0 && sizeof(R) == 4;
     __device__ __forceinline__ void reset_matrix() {
-        if constexpr (kLean) {
-            ident = true;
-        } else if (!LB) {
-            for (size_t e = threadIdx.x; e < (size_t)n * ldh; e += NT) {
-                const int i = (int)(e / ldh), j = (int)(e - (size_t)i * ldh);
-                mat[e] = i == j ? R(1) : R(0);
-            }
-            if (!MSM) fence_proxy_async_global();
-        }
+        if (!LB) ident = true;
     }
 
     // restart from steepest descent: identity H / empty history, direction -g
@@ -1568,9 +1560,9 @@ struct Opt {
                 }
                 if (!LB) {
                     __syncthreads();
-                    if constexpr (kLean) {
-                        if (ident) hpass_identity(pending);
-                        else if (MSM) hpass_rows4(pending);
+                    if (ident) hpass_identity(pending);
+                    else if constexpr (kLean) {
+                        if (MSM) hpass_rows4(pending);
                         else hpass_stream_v4(pending);
                     } else if (MSM) hpass(pending);
                     else hpass_stream(pending);
