@@ -220,9 +220,10 @@ __device__ void dg_gradient(const Args &a, const float4 *X, float4 *G, int mol, 
         const float4 xi = X[i];
         float gx = 0.f, gy = 0.f, gz = 0.f, gw = 0.f;
         const int e1 = __ldg(b.dinc_starts + r + 1);
-        // not unrolled: twice costs 2 % at 32 threads (246 vs 240 us, 10000 conformers of 18-48 atoms x 2
-        // iterations on B200), four times 15 % (registers, and instruction fetch between the branches)
-#pragma unroll 1
+        // one warp per conformer: not unrolled (246 -> 240 us, 10000 conformers of 18-48 atoms x 2
+        // iterations on B200); more warps: twice (1 % faster); four times is 8 to 15 % slower everywhere
+        // (registers, and instruction fetch between the branches)
+#pragma unroll (NT == 32 ? 1 : 2)
         for (int e = __ldg(b.dinc_starts + r); e < e1; ++e) {
             const float4 q = __ldg(inc + e);
             const float4 xo = X[__float_as_int(q.x)];
