@@ -132,8 +132,8 @@ int plan_minimize(const MMFFBatchDev *b, const MMFFConfDev *c, const MMFFOptPara
     if (fit < 0) return fit;
     // mixed-precision L-BFGS with the history in shared memory: the register-capped instance
     // (128 registers a thread) where two of its CTAs fit an SM by shared memory -- measured on
-    // the 150-170-atom class; where only one fits, the cap only adds spills (170-400 atoms
-    // measured 25 % slower).  Decided at the atom bound with a 32-entry class table (the
+    // the 150-170-atom class; where only one fits, the cap gains no CTA (170-400 atoms were
+    // 25 % slower, measured when the capped instance still spilled).  Decided at the atom bound with a 32-entry class table (the
     // serving classes' bound), so the instance does not depend on the launch's molecules; a
     // launch whose tables are larger still runs, with the CTAs that fit.
     if (mixed && lb && o->threads == 0) {

@@ -137,7 +137,7 @@ __device__ __forceinline__ int claim_slot(const Params &P) {
 __host__ __device__ __forceinline__ size_t al16(size_t x) { return (x + 15) & ~(size_t)15; }
 
 // Shared-memory layout of one CTA (byte offsets).
-constexpr int kStages = 4;         // rows of H in flight per warp (TMA ring)
+constexpr int kStages = 4;         // rows of H in flight per warp (TMA ring), two to a copy
 
 struct Layout {
     size_t pos4, pos4d, x, g, dir, xo, dg, hp, hq, pxi, pc, pr, gbuf, cls, q, mask, tab, red, rho, alpha,
