@@ -212,7 +212,8 @@ def load():
 
 class MappedHostArray:
     """A zeroed numpy array in host memory that the device can write (mmffb_host_alloc_mapped);
-    ``device_ptr`` is its device address.  Freed with the object."""
+    ``device_ptr`` is its device address.  Freed by ``free`` or with the object; the driver holds
+    that call until the device is idle, so an owner that knows when it is frees it then."""
 
     def __init__(self, n: int, dtype):
         import numpy as np
@@ -226,13 +227,17 @@ class MappedHostArray:
         buf = (ctypes.c_char * (max(1, n) * self.dtype.itemsize)).from_address(self._host)
         self.array = np.frombuffer(buf, dtype=self.dtype, count=max(1, n))
 
-    def __del__(self):
-        if getattr(self, "_host", None):
+    def free(self) -> None:
+        """Give the memory back (no launch that writes it may be running; ``array`` is gone)."""
+        host, self._host, self.array, self.device_ptr = getattr(self, "_host", None), None, None, 0
+        if host:
             try:
-                load().mmffb_host_free(self._host)
+                load().mmffb_host_free(host)
             except Exception:
                 pass
-            self._host = None
+
+    def __del__(self):
+        self.free()
 
 
 def check(rc: int, what: str) -> None:

@@ -713,6 +713,13 @@ class MMFFServer:
                     cs.copy_stream.synchronize()
                     for st in cs.streams:
                         st.synchronize()
+                # given back here, where no worker runs: left to the garbage collector, the call
+                # waited out whatever worker of a later server was running then (5 s measured, in
+                # that server's preparation)
+                for cs in self.classes.values():
+                    for h in cs.halves:
+                        h.done_np, h.done_dev = None, 0
+                        h.done_buf.free()
                 break
             time.sleep(0.0002)
 
