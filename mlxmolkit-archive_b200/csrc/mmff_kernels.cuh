@@ -526,8 +526,10 @@ __device__ __forceinline__ A eval_terms32(const Params &P, const MolV &m, const 
     // The warp's first chunk of a term type.  With gradients chunk c is warp c mod NW's, whose buffer
     // sums a fixed sequence; an energy alone deals the chunks of all types in one round, so that a
     // small molecule's few chunks do not all fall to the first warps (2500 conformers of 23-72 atoms x 5
-    // iterations: 1.28 -> 1.25 ms on B200).
-    const auto first = [&](int before) { return G ? warp : (warp + NW - before % NW) % NW; };
+    // iterations: 1.28 -> 1.25 ms on B200).  That orders the sum anew: 1e-16 of it with FP64 sums, but
+    // in FP32 some ulps of the total, which the line search would take for a change of energy, so
+    // FP32 sums keep the one deal.
+    const auto first = [&](int before) { return G || sizeof(A) == 4 ? warp : (warp + NW - before % NW) % NW; };
     const int anch0 = m.bnch, snch0 = anch0 + m.anch, onch0 = snch0 + m.snch, tnch0 = onch0 + m.onch;
 
     for (int c = first(0); c < m.bnch; c += NW) {
@@ -883,7 +885,8 @@ struct Opt {
         return sum(eval_terms<R, A, NW, true, sizeof(R) == 4>(P, m, pos4, gbuf, ms, nv, first ? kFirst : t32::kFused));
     }
 
-    // Energy alone in the instance's term precision (the bits of evaluate()'s energy).
+    // Energy alone in the instance's term precision: the same terms to the last bit as evaluate()'s.
+    // FP32 sums add them in the same order too (the same bits); FP64 sums in another (1e-16 apart).
     __device__ __forceinline__ A energy() {
         return sum(eval_terms<R, A, NW, false, sizeof(R) == 4>(P, m, pos4, gbuf, ms, nv));
     }

@@ -5,9 +5,10 @@
 // conformer's whole run follows from the last bit of each term.  Left to the compiler, whether a
 // product is fused with the sum it enters depends on the code around it: the same source line
 // gave other bits in an energy-only evaluation than in one with gradients, and in one kernel
-// instance than in another.  Here each product, sum and fused step is explicit, so an energy is
-// the same number whichever evaluation it comes from (a trial's energy may come with or without
-// its gradient), and code around the terms can change without changing results.
+// instance than in another.  Here each product, sum and fused step is explicit, so a term's energy
+// is the same number whichever evaluation it comes from (a trial's energy may come with or without
+// its gradient), and code around the terms can change without changing results.  (A conformer's
+// energy is the same number where its terms are also summed in the same order: see eval_terms32.)
 //
 // Conventions: a b + c d + e f is fma(e, f, fma(a, b, c d)) and a b - c d is fma(a, b, -(c d)).
 #pragma once
