@@ -30,8 +30,14 @@ struct MMArgs {
     int nv;                    // history row stride
 };
 
+// 16 warps an SM at 128 registers a thread: left to itself the compiler takes 168 in the 64-thread
+// instance, six CTAs an SM instead of eight, and the batches that instance is for -- more conformers
+// than the larger ones hold -- take more waves (1184 conformers of about 30 atoms x 30 iterations:
+// 1.39 ms against 0.95).  Launches that fit anyway, or that shared memory limits, run 1 to 3 % longer
+// capped; a fixed 64 threads on a few large molecules up to 13 % (still 10 % less than the serial
+// block sums took).
 template <int NT>
-__global__ void __launch_bounds__(NT) multimol_kernel(const MMArgs a) {
+__global__ void __launch_bounds__(NT, 512 / NT) multimol_kernel(const MMArgs a) {
     constexpr int NW = NT / 32;
     extern __shared__ __align__(16) unsigned char smem[];
     const Params &P = a.P;

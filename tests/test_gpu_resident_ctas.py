@@ -12,6 +12,7 @@ import pytest
 from mlxmolkit_b200 import _lib
 from mlxmolkit_b200 import mmff_minimize as mm
 from mlxmolkit_b200 import synth
+from mlxmolkit_b200.mmff_metal_optimizer import _MultiMolRun
 from mlxmolkit_b200.mmff_params import extract_mmff_params
 
 pytestmark = pytest.mark.gpu
@@ -61,3 +62,22 @@ def _fused_sd_ms(per_sm):
 
 def test_steepest_descent_holds_four_conformers_an_sm():
     assert _fused_sd_ms(4) < 1.5 * _fused_sd_ms(3)
+
+
+def _multi_mol_ms(per_sm):
+    import torch
+    m, x = _fill(per_sm)
+    run = _MultiMolRun(m, x, 10, 0.1, 0.3, 1e-4, threads=64)
+    start = torch.from_numpy(x).cuda()
+
+    def f():
+        run.x.copy_(start)
+        run.hcount.zero_()
+        run.converged.zero_()
+        run.step(_lib.MM_START, 0, 0, 100)
+        run.step(_lib.MM_RUN, 30, 30, 100)
+    return _ms(f)
+
+
+def test_multi_mol_with_64_threads_holds_eight_conformers_an_sm():
+    assert _multi_mol_ms(8) < 1.5 * _multi_mol_ms(6)
