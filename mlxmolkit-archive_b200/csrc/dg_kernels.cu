@@ -385,19 +385,25 @@ __device__ float etk_energy(const Args &a, const float4 *X, int mol, float *buf)
     return bsum<NT>(e, buf);
 }
 
-// Lanes that share an atom's incidence lists in the ETK gradient (a power of two up to 8): the count
-// with the least steps, rounds of atoms times list steps, a round costing about 1.5 steps more for
-// its shuffles.  One lane per atom left most of a block idle (50 atoms, 128 threads) or a second
-// round nearly empty (33-48 atoms, 32 threads), and the list, one dependent load after another, is
-// what the gradient waits for.  B200, 1000 conformers of 23-80 atoms x 2 ETK iterations: 169 ->
-// 143 us.  (The DG gradient keeps one lane per atom: shared lists gave it 3 %.)
+// Lanes that share an atom's incidence lists in the ETK gradient: two, four or eight, the count
+// with the least steps -- rounds of atoms times list steps, a round costing 2.5 steps more for its
+// shuffles and barrier, a step of four lanes 5 % and of two 15 % more than one of eight.  The list,
+// one dependent load after another, is what the gradient waits for.  One lane per atom left most of a
+// block idle or a second round nearly empty (B200, 1000 conformers of 23-80 atoms x 2 ETK iterations:
+// 169 -> 143 us shared), and is behind at every size measured even where its one round is full:
+// neighbouring lanes read neighbouring records, and a warp waits for the longest of fewer lists.
+// 6000 conformers x 10 iterations: 49 atoms on 64 threads 1.70 ms with one lane, 1.67 with two, 1.60
+// with eight (1.63 before lanes shared at all); 100 atoms on 128 threads 4.46, 4.26 and 4.00 (4.28).
+// Over 11-135 atoms on 32-256 threads the rule is 0.1 % from the best count on average, 2 % at the
+// most.  (The DG gradient keeps one lane per atom: shared lists gave it 3 %.)
 template <int NT>
 __device__ __forceinline__ int gradient_lanes(int N, int list) {
-    int best = 1;
+    int best = 2;
     float least = 3.4e38f;
 #pragma unroll
-    for (int g = 1; g <= 8; g *= 2) {
-        const float cost = (float)((N * g + NT - 1) / NT) * ((float)((list + g - 1) / g) + (g > 1 ? 1.5f : 0.0f));
+    for (int g = 2; g <= 8; g *= 2) {
+        const float step = g == 2 ? 1.15f : (g == 4 ? 1.05f : 1.0f);
+        const float cost = (float)((N * g + NT - 1) / NT) * ((float)((list + g - 1) / g) + 2.5f) * step;
         if (cost < least) {
             least = cost;
             best = g;
