@@ -538,9 +538,10 @@ def main():
                          "algorithmic_bytes_per_launch": abytes, "size_classes": bins,
                          "duration": "own kernel" if top_first else "upper bound (includes waiting for SMs)",
                          "peak_source": "MEASURED_PEAKS.json hbm_gbs (measured)" if peaks else "fallback",
-                         "note": "algorithmic bytes = 8n^2 + 40n + term bytes + 24N per iteration, term bytes "
-                                 "+ 12N per line-search evaluation (n = 3N); traffic scaled from an ncu capture "
-                                 "of a smaller case of the same kernel"},
+                         "note": "algorithmic bytes = term bytes + 12N per line-search trial, 40n + 12N per "
+                                 "iteration, 8n^2 per inverse-Hessian pass (n = 3N; none for the identity's, "
+                                 "4n^2 where its first update is written; L-BFGS 16n a history pair + 8n); "
+                                 "traffic scaled from an ncu capture of a smaller case of the same kernel"},
             "cpu_baseline": cpu, "plain_gpu_path": plain,
             "clocks": clk.summary(), "gpu_launches": a.steps * len(m.bins),
         }

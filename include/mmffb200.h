@@ -166,7 +166,8 @@ size_t mmffb_minimize_scratch_bytes(const MMFFBatchDev *batch, const MMFFConfDev
  * mmff_minimize_nk (mlxmolkit/mmff_minimize.py:231-346;
  * mmff_bfgs_source_tg.metal, mmff_lbfgs_source_tg.metal).
  * energy: float64[n_conf]; status, iters: int32[n_conf]; ls_evals (may be
- * NULL): int32[n_conf] energy-only line-search evaluations per conformer.
+ * NULL): int32[n_conf] line-search trials per conformer, each an energy with or
+ * without its gradient.
  */
 int mmffb_minimize(const MMFFBatchDev *batch, const MMFFConfDev *confs, const MMFFOptParams *opt,
                    float *pos, double *energy, int32_t *status, int32_t *iters, int32_t *ls_evals,

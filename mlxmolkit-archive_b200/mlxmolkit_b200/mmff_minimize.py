@@ -241,9 +241,9 @@ class Minimizer:
         """Minimise in place on the device; returns (energy, status, iters) device tensors.
 
         ``evals`` (optional int32 device tensor, one per conformer) receives the
-        number of energy-only line-search evaluations; ``err`` (optional int32
-        device tensor of one element) is set to 1 if a bounded wait inside the
-        kernel gave up (its conformers then have status ``ST_TIMEOUT``).
+        number of line-search trials; ``err`` (optional int32 device tensor of one
+        element) is set to 1 if a bounded wait inside the kernel gave up (its
+        conformers then have status ``ST_TIMEOUT``).
         """
         torch = _torch()
         L = _lib.load()

@@ -1,4 +1,4 @@
-"""Algorithmic bytes of a dense-BFGS minimisation, the numerator of the HBM roofline."""
+"""Algorithmic bytes of a minimisation, the numerator of the HBM roofline."""
 from __future__ import annotations
 
 import numpy as np
@@ -12,20 +12,29 @@ def term_bytes(p) -> int:
 
 
 def algorithmic_bytes(params, conf_mol, iters, evals, history_m: int = 0) -> float:
-    """Algorithmic HBM bytes of minimising the conformers ``conf_mol`` (molecule indices).
+    """Algorithmic HBM bytes of minimising the conformers ``conf_mol`` (molecule indices): what
+    ``iters`` iterations with ``evals`` line-search trials cannot do without.
 
-    Per iteration of dense BFGS (history_m == 0): the inverse Hessian read and
-    written once (4-byte elements, 8 n^2 for n = 3N coordinates).  Per iteration
-    of L-BFGS: the two-loop recursion's reads of S and Y twice (16 m n) and the
-    new pair (8 n).  Either way, 40 n for the BFGS vectors, the term records and
-    24 B per atom of coordinates and gradient.  Per energy-only line-search
-    evaluation: the term records and 12 B per atom.
+    The term records and 12 B per atom of coordinates once for the start and once per trial (the
+    accepted trial's evaluation is also the next iteration's gradient); 12 B per atom of gradient for
+    the start and per iteration; 40 n for the vectors per iteration (n = 3N coordinates).  Between
+    iterations, dense BFGS (history_m == 0): nothing while the inverse Hessian is the identity
+    (the first pass), 4 n^2 where its first update is written, 8 n^2 in each later pass (4-byte
+    elements read and written once).  L-BFGS: the two-loop recursion's reads of the S and Y held so far
+    twice (16 n a pair) and the new pair (8 n).  Not counted, though run: the second evaluation of a
+    trial that was evaluated without its gradient and then accepted, that of a failed search's
+    point, and a restart's passes are taken for ordinary ones.
     """
     conf_mol = np.asarray(conf_mol)
+    it, ev = np.asarray(iters, np.float64), np.asarray(evals, np.float64)
     n_atoms = np.array([p.n_atoms for p in params], dtype=np.float64)[conf_mol]
     tb = np.array([term_bytes(p) for p in params], dtype=np.float64)[conf_mol]
     n = 3 * n_atoms
-    quasi = 16 * history_m * n + 8 * n if history_m > 0 else 8 * n * n
-    per_iter = quasi + 40 * n + tb + 24 * n_atoms
-    per_eval = tb + 12 * n_atoms
-    return float(np.sum(np.asarray(iters, np.float64) * per_iter + np.asarray(evals, np.float64) * per_eval))
+    passes = np.maximum(it - 1, 0)
+    if history_m > 0:
+        filling = np.minimum(passes, history_m)
+        pairs = filling * (filling + 1) / 2 + (passes - filling) * history_m
+        quasi = 16 * n * pairs + 8 * n * passes
+    else:
+        quasi = 4 * n * n * np.maximum(2 * passes - 3, 0)
+    return float(np.sum(quasi + (1 + ev) * (tb + 12 * n_atoms) + (1 + it) * 12 * n_atoms + it * 40 * n))
