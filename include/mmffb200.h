@@ -114,7 +114,9 @@ typedef struct {
     int32_t give_up_waits;       /* test switch, 0 in normal use: 1 = every wait for a row copy gives up
                                     before testing, as if the copy never completed, which exercises the
                                     timeout path (the kernel drains the copies in flight, its conformers
-                                    end MMFFB_ST_TIMEOUT and the error word is set) */
+                                    end MMFFB_ST_TIMEOUT and the error word is set; the first two passes,
+                                    an identity's, wait for nothing, so a run that ends within them is
+                                    a normal one) */
     int32_t *err_word;           /* optional device int32, zeroed by the call; 1 once the launch is done
                                     if a bounded wait gave up (the affected conformers then have status
                                     MMFFB_ST_TIMEOUT).  With or without it, mmffb_minimize's scratch

@@ -277,10 +277,8 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
     return r;
 }
 
-template <class R> __device__ __forceinline__ R qprod(double a, double b);
-template <> __device__ __forceinline__ float qprod<float>(double a, double b) { return (float)(a * b); }
 // the term lists carry q_i*q_j rounded to float32 (mmff_params.py:305,318); every precision uses it
-template <> __device__ __forceinline__ double qprod<double>(double a, double b) { return (double)(float)(a * b); }
+__device__ __forceinline__ double qprod(double a, double b) { return (double)(float)(a * b); }
 
 template <class T> __device__ __forceinline__ T wsum(T v) {
 #pragma unroll
@@ -373,10 +371,6 @@ struct MolSmem {
 
 template <class R> __device__ __forceinline__ void ld3(const R *p4, int a, R &x, R &y, R &z) {
     x = p4[4 * a]; y = p4[4 * a + 1]; z = p4[4 * a + 2];
-}
-template <> __device__ __forceinline__ void ld3<float>(const float *p4, int a, float &x, float &y, float &z) {
-    const float4 v = reinterpret_cast<const float4 *>(p4)[a];
-    x = v.x; y = v.y; z = v.z;
 }
 
 // The class table's row of the class at offset cls8, and the row's entry of another.
@@ -769,7 +763,7 @@ __device__ __forceinline__ A eval_terms(const Params &P, const MolV &m, const R 
                 const int cj = ms.cls[j];
                 const float2 t1 = table_at(ti, cj), t2 = table_at(tk, cj);
                 const uint32_t w14 = wi.y, w14b = wk.y;
-                R q1 = qprod<R>(ms.qa[i], ms.qa[j]), q2 = qprod<R>(ms.qa[ik], ms.qa[j]);
+                R q1 = qprod(ms.qa[i], ms.qa[j]), q2 = qprod(ms.qa[ik], ms.qa[j]);
                 if ((w14 >> lane) & 1u) q1 *= R(0.75);
                 if ((w14b >> lane) & 1u) q2 *= R(0.75);
                 R xj, yj, zj;

@@ -22,9 +22,9 @@ struct TermMode {
 };
 
 template <class R> struct Num;
-// FP32: hardware approximate reciprocal / reciprocal square root (about 2 ulp); the
-// FP32 paths are checked against the FP64 oracle to 1e-5 relative, and the line
-// search of the mixed path switches to FP64 energies near convergence.
+// FP32: hardware approximate reciprocal / reciprocal square root (about 2 ulp).  Only the
+// plain path (mmff_plain.cu) evaluates its FP32 terms with these functions; the
+// others use mmff_terms32.cuh.
 template <> struct Num<float> {
     static __device__ __forceinline__ float sqrt_(float x) { return x * rsqrtf(x); }   // x > 0 here
     static __device__ __forceinline__ float rsqrt_(float x) { return rsqrtf(x); }

@@ -86,8 +86,10 @@ __device__ __forceinline__ void accm(float *dst, float s, const V3 &v) {
 }
 
 // Three steps of the gradient have two forms.  A run's first gradient has always been rounded
-// with the product set apart in them, the later ones with it fused; both are kept, so that runs
-// keep their results bit for bit.
+// with the product set apart in them (the stretch-bend's only in the 128-register L-BFGS instance
+// with its history in shared memory), the later ones and every other caller's with it fused; both are
+// kept, so that runs keep their results bit for bit.  A run's first gradient therefore differs from
+// an energy_grad call's at the same point in its last bits.
 enum Forms { kFused = 0, kBondApart = 1, kTorsionApart = 2, kStrbendApart = 4 };
 
 // 1 - c^2
