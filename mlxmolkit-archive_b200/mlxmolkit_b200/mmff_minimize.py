@@ -69,7 +69,7 @@ def _upload(arrays, device):
     boundary (the bonded records' alignment): one buffer and one copy for all the small ones, a copy
     from where it is for each large one."""
     torch = _torch()
-    arrays = [np.require(a, requirements="CW").reshape(-1) for a in arrays]
+    arrays = [np.ascontiguousarray(a).reshape(-1) for a in arrays]
     starts, end = [], 0
     for a in arrays:
         starts.append(end)
@@ -81,7 +81,8 @@ def _upload(arrays, device):
             host[o:o + a.nbytes] = a.view(np.uint8)
     dev = torch.from_numpy(host).to(device, non_blocking=False)
     return [dev[o:o + a.nbytes].view(getattr(torch, a.dtype.name)) if a.nbytes <= _JOIN_BYTES
-            else torch.from_numpy(a).to(device, non_blocking=False) for a, o in zip(arrays, starts)]
+            else torch.from_numpy(a if a.flags.writeable else a.copy()).to(device, non_blocking=False)
+            for a, o in zip(arrays, starts)]
 
 
 class DeviceBatch:

@@ -51,3 +51,12 @@ def test_no_arrays_and_empty_arrays():
     (t,) = mm._upload([np.zeros(0, np.int64)], torch.device("cpu"))
     assert t.numel() == 0 and t.dtype == torch.int64
 
+
+
+@pytest.mark.filterwarnings("error")
+def test_read_only_arrays_go_up_too():
+    a = [np.zeros(4, np.float32), np.ones(LARGE, np.float32)]
+    for x in a:
+        x.flags.writeable = False
+    out = mm._upload(a, torch.device("cpu"))
+    assert out[0].sum() == 0 and out[1].sum() == LARGE
