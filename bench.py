@@ -263,8 +263,8 @@ def _dg_main(a, rank: int, world: int):
         "converged_frac": conv,
         "e2e": {"value": C / t_e2e, "unit": UNIT, "h2d_bytes_per_step": 2 * nbytes, "d2h_bytes_per_step": 2 * nbytes + 16 * C},
         "roofline": None,
-        "roofline_note": "latency-bound, not HBM or tensor (profiles/dg_minimize_kernel_20x50.md: 2.9 MB of DRAM "
-                         "traffic in a 61 ms launch, 23.5 % issue active)",
+        "roofline_note": "latency-bound, not HBM or tensor (profiles/dg_minimize_kernel_20x50.md: 3.1 MB of DRAM "
+                         "traffic in a 50 ms launch, 26.8 % issue active)",
         "cpu_baseline": {"value": ns / dt_cpu, "unit": UNIT, "cores": cores, "kind": "port",
                          "sample": f"{ns} seeded conformers of the workload, FP64 DG L-BFGS + collapse "
                                    f"(oracle/dg_oracle.c), converged {conv_cpu:.3f}"},
@@ -462,7 +462,8 @@ def main():
         # DRAM bytes per algorithmic byte of this kernel, from an ncu capture of a
         # smaller case of the same size class, scaled to this launch
         tr = json.load(open(os.path.join(ROOT, "profiles", "minimize_kernel_traffic.json")))
-        traffic = float(tr["dram_bytes_per_algorithmic_byte"]) * abytes
+        if not hist:        # the captured kernel is the dense one
+            traffic = float(tr["dram_bytes_per_algorithmic_byte"]) * abytes
     except (OSError, ValueError, KeyError):
         pass
 
