@@ -133,9 +133,10 @@ int plan_minimize(const MMFFBatchDev *b, const MMFFConfDev *c, const MMFFOptPara
     // mixed-precision L-BFGS with the history in shared memory: the register-capped instance
     // (128 registers a thread) where two of its CTAs fit an SM by shared memory -- measured on
     // the 150-170-atom class; where only one fits, the cap gains no CTA (170-400 atoms were
-    // 25 % slower, measured when the capped instance still spilled).  Decided at the atom bound with a 32-entry class table (the
-    // serving classes' bound), so the instance does not depend on the launch's molecules; a
-    // launch whose tables are larger still runs, with the CTAs that fit.
+    // 25 % slower, measured when the capped instance still spilled).  Decided at the atom bound
+    // with a 32-entry class table (the serving classes' bound), so the instance does not depend
+    // on the launch's molecules; a launch whose tables are larger still runs, with the CTAs that
+    // fit.
     if (mixed && lb && o->threads == 0) {
         // the register-capped instance with the history where it is: in shared memory if two
         // CTAs fit so, else in a global slot if two fit that way (up to about 290 atoms; the
